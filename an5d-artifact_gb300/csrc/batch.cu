@@ -17,9 +17,8 @@
 //
 // Memory ordering: a finishing item's lanes fence their stores, then lane 0
 // increments its block's counter; a starting item's lane 0 reads the
-// counters with acquire semantics and issues a proxy fence before its bulk
-// copies (an async-proxy read) touch the data. Loads outside the bulk copies
-// bypass L1.
+// counters with acquire semantics before the warp's copies touch the data
+// (cp.async.cg and the other loads of a grid bypass L1).
 //
 // Built twice: -DGBS_FMA=0 (exact mode) and -DGBS_FMA=1.
 #include <cuda_runtime.h>
@@ -64,7 +63,7 @@ using batchdetail::Item;
 
 namespace {
 constexpr bool kFma = GBS_FMA != 0;
-constexpr int kWpc = kWpc2D, kStages = kStages2D;
+constexpr int kWpc = kWpc2D;
 // CTAs per SM the batched kernels are built for. The layered kernel takes 4
 // (at most 128 registers a thread, 16 warps an SM; every variant but
 // star2d3r at degree 2 fits without spilling): 2.92x the per-grid launches
@@ -111,13 +110,11 @@ static_assert(sizeof(Params2D<float, batchdetail::kMaxTerms>) <= kParamSlot, "pa
 // forces a local-memory frame onto every variant's loop) and the call costs
 // once per item. The parameters (with up to 81 coefficients) are staged in
 // shared memory: a per-thread copy would sit on the local-memory stack.
-// Everything else comes by value (time block k, strip, stream block, the
-// warp's copy count) and the new copy count is the return value, ~0u when a
-// bounded wait gave up: a reference into the caller's frame would place
-// that frame in local memory.
+// Everything else comes by value (time block k, strip, stream block): a
+// reference into the caller's frame would place that frame in local memory.
 template <class S, int B>
-__device__ __noinline__ unsigned run_item(const GridDev *gp, int k, int strip, int blk, float *ring,
-                                          uint64_t *bars, unsigned load_base, int *err, unsigned char *slot) {
+__device__ __noinline__ void run_item(const GridDev *gp, int k, int strip, int blk, unsigned char *ring,
+                                      unsigned char *slot) {
   const GridDev &g = *gp;
   auto &p = *reinterpret_cast<Params2D<float, S::kTerms> *>(slot);
   const int lane = threadIdx.x & 31;
@@ -125,13 +122,10 @@ __device__ __noinline__ unsigned run_item(const GridDev *gp, int k, int strip, i
   if (lane == 0) {
     p.src = g.base + (long long)(k % 2) * g.plane;
     p.dst = g.base + (long long)((k + 1) % 2) * g.plane;
-    p.err = err;
     p.pitch = g.pitch;
     p.d0 = g.d0;
     p.d1 = g.d1;
     p.shift = g.shift;
-    p.b = B;
-    p.wout = ((128 - 2 * B * S::kRad - 3) / 4) * 4;
     p.nstrips = 0;
     p.nblocks = g.nblocks;
     p.sl = g.sl;
@@ -143,53 +137,63 @@ __device__ __noinline__ unsigned run_item(const GridDev *gp, int k, int strip, i
     p.stash_stride = 0;
   }
   __syncwarp();
-  bool ok;
   if constexpr (S::kTerms <= 25) {
     // small parameter sets ride in registers for the whole item
     const Params2D<float, S::kTerms> pl = p;
-    ok = warp_item2d<S, float, B, kFma, kStages>(pl, strip, blk, ring, bars, load_base);
+    warp_item2d<S, float, B, kFma>(pl, strip, blk, ring);
   } else {
-    ok = warp_item2d<S, float, B, kFma, kStages>(p, strip, blk, ring, bars, load_base);
+    warp_item2d<S, float, B, kFma>(p, strip, blk, ring);
   }
   __syncwarp();  // the slot is rewritten by the next item
-  return ok ? load_base : ~0u;
 }
 
 template <class S>
-__device__ __forceinline__ bool dispatch_b(const GridDev &g, const Item &it, float *ring, uint64_t *bars,
-                                           unsigned &load_base, int *err, unsigned char *slot) {
+__device__ __forceinline__ void dispatch_b(const GridDev &g, const Item &it, unsigned char *ring,
+                                           unsigned char *slot) {
   constexpr int BS = batch_degree<S>();
-  unsigned next = ~0u;
-  if (it.b == BS) next = run_item<S, BS>(&g, it.k, it.strip, it.blk, ring, bars, load_base, err, slot);
+  if (it.b == BS) run_item<S, BS>(&g, it.k, it.strip, it.blk, ring, slot);
   if constexpr (BS != 1) {
-    if (it.b == 1) next = run_item<S, 1>(&g, it.k, it.strip, it.blk, ring, bars, load_base, err, slot);
+    if (it.b == 1) run_item<S, 1>(&g, it.k, it.strip, it.blk, ring, slot);
   }
-  if (next == ~0u) return false;
-  load_base = next;
-  return true;
 }
 
-__device__ __forceinline__ bool dispatch(const GridDev &g, const Item &it, float *ring, uint64_t *bars,
-                                         unsigned &load_base, int *err, unsigned char *slot) {
+__device__ __forceinline__ void dispatch(const GridDev &g, const Item &it, unsigned char *ring, unsigned char *slot) {
   switch (g.sid) {
 #define GBS_CASE(id, S)                                                  \
   case id:                                                               \
-    if constexpr (S::kDim == 2)                                          \
-      return dispatch_b<S>(g, it, ring, bars, load_base, err, slot);     \
-    else                                                                 \
-      return false;
+    if constexpr (S::kDim == 2) dispatch_b<S>(g, it, ring, slot);        \
+    break;
     GBS_FOR_EACH_STENCIL(GBS_CASE)
 #undef GBS_CASE
     default:
-      return false;
+      break;
   }
 }
 
+// shared memory of one warp: the largest ring of any variant the dispatcher runs
+template <class S> constexpr unsigned ring_bytes() {
+  if constexpr (S::kDim != 2) return 0;
+  else {
+    constexpr unsigned a = Pipe2D<S, float, batch_degree<S>(), kFma>::RING, b = Pipe2D<S, float, 1, kFma>::RING;
+    return a > b ? a : b;
+  }
+}
+constexpr unsigned max_ring() {
+  unsigned m = 0;
+#define GBS_RING(id, S) m = ring_bytes<S>() > m ? ring_bytes<S>() : m;
+  GBS_FOR_EACH_STENCIL(GBS_RING)
+#undef GBS_RING
+  return m;
+}
+constexpr unsigned kRing = (max_ring() + 127) / 128 * 128;
+// shared memory of a CTA: its warps' rings, then their parameter slots
+constexpr size_t kBatchSmem = (size_t)kWpc * (kRing + kParamSlot);
+
 // One work item on one warp: wait (bounded) until the stream blocks it
 // reads have finished the grid's earlier time blocks, run it, count it done.
-// False when a wait gave up (the error word says which).
-__device__ __forceinline__ bool persistent_item(const Args &a, unsigned idx, float *ring, uint64_t *bars,
-                                                unsigned &load_base, unsigned char *slot) {
+// False when the wait gave up (the error word says so).
+__device__ __forceinline__ bool persistent_item(const Args &a, unsigned idx, unsigned char *ring,
+                                                unsigned char *slot) {
   const int lane = threadIdx.x & 31;
   const Item it = a.items[idx];
   bool ok = true;
@@ -215,14 +219,10 @@ __device__ __forceinline__ bool persistent_item(const Args &a, unsigned idx, flo
         }
       }
     }
-    asm volatile("fence.proxy.async.global;" ::: "memory");
   }
   if (!__all_sync(0xffffffffu, ok)) return false;
   __syncwarp();
-  if (!dispatch(g, it, ring, bars, load_base, a.err, slot)) {
-    if (lane == 0) atomicOr(a.err, ERR_WAIT_TIMEOUT);
-    return false;
-  }
+  dispatch(g, it, ring, slot);
   __threadfence();
   __syncwarp();
   if (lane == 0) atomicAdd(&a.done[cown], 1u);
@@ -242,12 +242,8 @@ __global__ void __launch_bounds__(kWpc * 32, kPersistentCtas) batch2d_kernel(con
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned s_group;
   __shared__ int s_stop;
-  float *ring;
-  uint64_t *bars;
-  warp_ring2d<float, kWpc, kStages>(smem_raw, ring, bars);
-  unsigned char *slot = smem_raw + (size_t)kWpc * kStages * (128 * sizeof(float) + sizeof(uint64_t)) +
-                        (size_t)(threadIdx.x >> 5) * kParamSlot;
-  unsigned load_base = 0;
+  unsigned char *ring = smem_raw + (size_t)(threadIdx.x >> 5) * kRing;
+  unsigned char *slot = smem_raw + (size_t)kWpc * kRing + (size_t)(threadIdx.x >> 5) * kParamSlot;
   if (threadIdx.x == 0) s_stop = 0;
   while (true) {
     if (threadIdx.x == 0) s_group = atomicAdd(a.next, 1u);
@@ -257,7 +253,7 @@ __global__ void __launch_bounds__(kWpc * 32, kPersistentCtas) batch2d_kernel(con
     __syncthreads();  // s_group and s_stop are read before they are written again
     if (stop) break;
     const unsigned idx = first + (threadIdx.x >> 5);
-    if (idx < (unsigned)a.nitems && !persistent_item(a, idx, ring, bars, load_base, slot) &&
+    if (idx < (unsigned)a.nitems && !persistent_item(a, idx, ring, slot) &&
         (threadIdx.x & 31) == 0)
       s_stop = 1;
   }
@@ -270,15 +266,10 @@ __global__ void __launch_bounds__(kWpc * 32, kLayerCtas) batch_layer_kernel(cons
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const long long gw = (long long)blockIdx.x * kWpc + (threadIdx.x >> 5);
   if (gw >= count) return;
-  float *ring;
-  uint64_t *bars;
-  warp_ring2d<float, kWpc, kStages>(smem_raw, ring, bars);
-  unsigned char *slot = smem_raw + (size_t)kWpc * kStages * (128 * sizeof(float) + sizeof(uint64_t)) +
-                        (size_t)(threadIdx.x >> 5) * kParamSlot;
-  unsigned load_base = 0;
+  unsigned char *ring = smem_raw + (size_t)(threadIdx.x >> 5) * kRing;
+  unsigned char *slot = smem_raw + (size_t)kWpc * kRing + (size_t)(threadIdx.x >> 5) * kParamSlot;
   const Item it = a.items[first + gw];
-  if (!dispatch(a.grids[it.grid], it, ring, bars, load_base, a.err, slot) && (threadIdx.x & 31) == 0)
-    atomicOr(a.err, ERR_WAIT_TIMEOUT);
+  dispatch(a.grids[it.grid], it, ring, slot);
 }
 
 // ---------------------------------------------------------------------------
@@ -427,7 +418,7 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
       if (grids[g].stencil != sid || k >= blocks[g].size()) continue;
       const int b = blocks[g][k];
       const gbs_stencil_def_t *s = stencil_def(grids[g].stencil);
-      const int wout = ((128 - 2 * b * s->rad - 3) / 4) * 4;
+      const int wout = wout2d(s->rad, b, 4);
       const int nj = gd[g].d1 - 2 * s->rad;
       const int nstrips = (nj + wout - 1) / wout;
       const int need = done_before[g];
@@ -459,7 +450,7 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
     gbs_batch_destroy(h);
     return st;
   }
-  h->smem = (size_t)kWpc * kStages * (128 * sizeof(float) + sizeof(uint64_t)) + (size_t)kWpc * kParamSlot;
+  h->smem = kBatchSmem;
   int per_sm = 0, dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -630,7 +621,7 @@ gbs_status run(const gbs_batch_grid *grids, int ngrids, cudaStream_t stream) {
         if (k >= full + single) continue;
         const int b = k < full ? bs : 1;
         const gbs_stencil_def_t *s = stencil_def(sid);
-        const int wout = ((128 - 2 * b * s->rad - 3) / 4) * 4;
+        const int wout = wout2d(s->rad, b, 4);
         const int nstrips = (h_grids[g].d1 - 2 * s->rad + wout - 1) / wout;
         const int count = nstrips * h_grids[g].nblocks;
         if (nitems + count > kMaxItems)
@@ -673,7 +664,7 @@ gbs_status run(const gbs_batch_grid *grids, int ngrids, cudaStream_t stream) {
   a.next = sc->counters;
   a.done = sc->counters + 1;
   a.err = &sc->err;
-  const size_t smem = (size_t)kWpc * kStages * (128 * sizeof(float) + sizeof(uint64_t)) + (size_t)kWpc * kParamSlot;
+  const size_t smem = kBatchSmem;
   int per_sm = 0, sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch2d_kernel, kWpc * 32, smem) != cudaSuccess ||

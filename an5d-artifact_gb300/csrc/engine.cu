@@ -240,24 +240,48 @@ long long resident_warps_2d(int sid, int dtype, int fma, int b) {
   return (long long)c * sm_count();
 }
 
+// Rows per stream block of a 2-D launch: the ones that the busiest SM gets
+// through first. A warp streams sl rows plus the overlap; the CTAs (one warp
+// per scheduler each) of an SM share its issue slots (float) or its FP64 pipe
+// (double); float needs about 3.3 CTAs to fill them (with fewer, a row costs
+// its own latency), double 2 (64 cycles of a scheduler's pipe per FP64
+// instruction hide the rest). So short blocks for grids that leave the chip idle (a 128x96 grid
+// in blocks of 16 rows spent its time streaming them one by one on two SMs),
+// and for larger ones as many CTAs on every SM as on the busiest.
+static int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps) {
+  const int sms = sm_count();
+  const int res = (int)std::max<long long>(1, (resident_warps > 0 ? resident_warps : 16LL * sms) /
+                                                  (kWarpsPerCta2D * (long long)sms));
+  const double alone = f64 ? 2.0 : 3.3;
+  const double overlap = 2.0 * br + 2.0;
+  double best = 1e300;
+  int best_sl = ni;
+  // more blocks than fill the chip 16 times over gain nothing
+  const long long most = std::min<long long>(ni, std::max<long long>(1, 16LL * sms * res * kWarpsPerCta2D / nstrips));
+  for (long long nb = 1; nb <= most; ++nb) {
+    const int sl = (int)((ni + nb - 1) / nb);
+    const long long ctas = ((ni + sl - 1) / sl * (long long)nstrips + kWarpsPerCta2D - 1) / kWarpsPerCta2D;
+    const long long per_sm = (ctas + sms - 1) / sms;
+    const long long full = per_sm / res, rem = per_sm % res;
+    const double cost =
+        (sl + overlap) * (full * std::max(alone, (double)res) + (rem ? std::max(alone, (double)rem) : 0.0));
+    if (cost < best) {
+      best = cost;
+      best_sl = sl;
+    }
+  }
+  return best_sl;
+}
+
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident) {
   Geometry2D g{};
-  const int R = L.rad, V = L.V;
+  const int R = L.rad;
   g.b = b;
-  // window starts are 16-byte aligned, so the strip can start up to V-1
-  // columns inside it
-  g.wout = ((32 * V - 2 * b * R - (V - 1)) / V) * V;
+  g.wout = wout2d(R, b, L.V);
   const int ni = L.dims[0] - 2 * R, nj = L.dims[1] - 2 * R;
   g.nstrips = g.wout > 0 ? (nj + g.wout - 1) / g.wout : 1;
   int sl = sl_req;
-  if (sl <= 0) {
-    // one full wave of resident warps, each streaming one block; blocks at
-    // least 4*b*r rows long so that the stream overlap stays small
-    if (resident <= 0) resident = 152LL * 16;
-    long long nb = std::max<long long>(1, resident / std::max(1, g.nstrips));
-    sl = (int)((ni + nb - 1) / nb);
-    sl = std::max(sl, std::max(8, 4 * b * R));
-  }
+  if (sl <= 0) sl = stream_rows_2d(g.nstrips, ni, b * R, L.esize == 8, resident);
   g.sl = std::min(sl, ni);
   g.nblocks = (ni + g.sl - 1) / g.sl;
   return g;
@@ -369,9 +393,11 @@ gbs_status validate3d(const Layout &L, const Geometry3D &g) {
   return GBS_OK;
 }
 
-// Every address range a 2-D launch touches, checked against the buffer.
+// The column windows of a 2-D launch, checked against the grid. (A window may
+// reach past the padded row: the kernel's copies are guarded per vector, and
+// it stores interior columns only.)
 gbs_status validate2d(const Layout &L, const Geometry2D &g) {
-  const int R = L.rad, V = L.V, ROW = 32 * V;
+  const int R = L.rad, V = L.V;
   if (g.wout <= 0) return fail(GBS_ERR_UNSUPPORTED, "fused degree %d leaves no output columns", g.b);
   if (L.shift % 1 != 0 || (L.pitch * (long long)L.esize) % 16 != 0)
     return fail(GBS_ERR_INVALID, "internal: row pitch not 16-byte aligned");
@@ -380,11 +406,9 @@ gbs_status validate2d(const Layout &L, const Geometry2D &g) {
     const int ce = std::min(cs + g.wout, L.dims[1] - R);
     const int need_lo = std::max(0, cs - g.b * R);
     const int need_hi = std::min(L.dims[1], ce + g.b * R);
-    const long long ws = ((need_lo + L.shift) / V) * (long long)V;
-    if (ws < 0 || ws + ROW > L.pitch)
-      return fail(GBS_ERR_INVALID, "internal: strip %d window [%lld,%lld) outside row of %lld", s, ws,
-                  ws + ROW, L.pitch);
-    if (need_hi + L.shift > ws + ROW)
+    const int left = (g.b * R + V - 1) / V * V;
+    const long long ws = (long long)cs + L.shift - left;
+    if (need_lo + L.shift < ws || need_hi + L.shift > ws + 32 * V || need_hi + L.shift > L.pitch)
       return fail(GBS_ERR_INVALID, "internal: strip %d window misses columns", s);
     if ((ws * (long long)L.esize) % 16 != 0) return fail(GBS_ERR_INVALID, "internal: unaligned window");
   }
@@ -489,17 +513,99 @@ gbs_status run_loop(const gbs_desc *d, const Layout &L, void *dev_A, cudaStream_
   const std::vector<int> steps = split_steps(d->timestep, bt);
   char *base = static_cast<char *>(dev_A);
   const size_t plane_bytes = (size_t)L.plane * L.esize;
+  BlockPlan plan;  // the steps come in one run of each degree
   for (size_t j = 0; j < steps.size(); ++j) {
-    gbs_status st = launch_block(d, L, coef.data(), div, eps, sl, steps[j], base + (j % 2) * plane_bytes,
-                                 base + ((j + 1) % 2) * plane_bytes, stream, err);
+    gbs_status st = GBS_OK;
+    if (j == 0 || steps[j] != steps[j - 1])
+      st = plan_block(d, L, coef.data(), div, eps, sl, steps[j], false, err, &plan);
+    // each launch but the first follows the previous one of this loop on the stream
+    if (st == GBS_OK)
+      st = launch_plan(plan, base + (j % 2) * plane_bytes, base + ((j + 1) % 2) * plane_bytes, nullptr, stream, j > 0);
     if (st != GBS_OK) return st;
   }
   return GBS_OK;
 }
 
+gbs_status plan_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl, int b,
+                      bool stash, int *err, BlockPlan *out) {
+  const gbs_stencil_def_t *s = stencil_def(d->stencil);
+  if (stash && s->dim != 2) return fail(GBS_ERR_UNSUPPORTED, "stashed launches take 2-D grids");
+  const int fma = d->fp_mode == GBS_FP_FMA ? 1 : 0;
+  const Picks &pk = picks(d->stencil, d->dtype, fma);
+  if (b < 1 || b > pk.maxb)
+    return fail(GBS_ERR_UNSUPPORTED, "no kernel of degree %d built for %s", b, s->name);
+  *out = BlockPlan{};
+  out->dim = s->dim;
+  if (s->dim == 2) {
+    Geometry2D g = geometry2d(L, b, sl, resident_warps_2d(d->stencil, d->dtype, fma, b));
+    gbs_status st = validate2d(L, g);
+    if (st != GBS_OK) return st;
+    Launch2D &a = out->a2;
+    a.pitch = L.pitch;
+    a.d0 = L.dims[0];
+    a.d1 = L.dims[1];
+    a.shift = (int)L.shift;
+    a.wout = g.wout;
+    a.nstrips = g.nstrips;
+    a.nblocks = g.nblocks;
+    a.sl = g.sl;
+    a.coef = coef;
+    a.div = div;
+    a.eps = eps;
+    a.div_proven = d->dtype == GBS_F32 && div_proven_exact(div);
+    a.stash_stride = L.plane;
+    out->f2 = stash ? pk.l2s[b] : pk.l2[b];
+    if (!out->f2) return fail(GBS_ERR_UNSUPPORTED, "no 2-D kernel%s for b=%d", stash ? " in stash mode" : "", b);
+  } else {
+    const int v = variant_3d(d, b);
+    if (v < 0) return GBS_ERR_UNSUPPORTED;
+    Geometry3D g = geometry3d(L, b, tile_shape_3d(d->stencil, d->dtype, fma, b, v), sl,
+                              resident_ctas_3d(d->stencil, d->dtype, fma, b, v));
+    gbs_status st = validate3d(L, g);
+    if (st != GBS_OK) return st;
+    Launch3D &a = out->a3;
+    a.err = err;
+    a.pitch = L.pitch;
+    a.d0 = L.dims[0];
+    a.d1 = L.dims[1];
+    a.d2 = L.dims[2];
+    a.shift = (int)L.shift;
+    a.b = b;
+    a.jout = g.jout;
+    a.wk = g.wk;
+    a.ntk = g.ntk;
+    a.ntj = g.ntj;
+    a.nblocks = g.nblocks;
+    a.sl = g.sl;
+    a.coef = coef;
+    a.div = div;
+    a.div_proven = d->dtype == GBS_F32 && div_proven_exact(div);
+    out->f3 = pk.l3[b][v];
+    if (!out->f3) return fail(GBS_ERR_UNSUPPORTED, "no 3-D kernel for b=%d", b);
+  }
+  return GBS_OK;
+}
+
+gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream, bool pdl) {
+  cudaError_t e;
+  if (plan.dim == 2) {
+    plan.a2.src = src;
+    plan.a2.dst = dst;
+    plan.a2.stash = stash;
+    plan.a2.pdl = pdl;
+    e = plan.f2(plan.a2, stream);
+  } else {
+    plan.a3.src = src;
+    plan.a3.dst = dst;
+    plan.a3.pdl = pdl;
+    e = plan.f3(plan.a3, stream);
+  }
+  return e == cudaSuccess ? GBS_OK : cuda_fail(e, plan.dim == 2 ? "2-D stencil launch" : "3-D stencil launch");
+}
+
 // One launch of b fused steps from plane src to plane dst (layout L; the
 // interior of dst is written, its halo never): coefficients as the source
-// writes them, divisor and eps resolved, sl 0 = one wave.
+// writes them, divisor and eps resolved, sl 0 = the planner's choice.
 gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                         int b, const void *src, void *dst, cudaStream_t stream, int *err) {
   return launch_block_stash(d, L, coef, div, eps, sl, b, src, dst, nullptr, stream, err);
@@ -507,72 +613,9 @@ gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, 
 
 gbs_status launch_block_stash(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                               int b, const void *src, void *dst, void *stash, cudaStream_t stream, int *err) {
-  const gbs_stencil_def_t *s = stencil_def(d->stencil);
-  if (stash && s->dim != 2) return fail(GBS_ERR_UNSUPPORTED, "stashed launches take 2-D grids");
-  const int fma = d->fp_mode == GBS_FP_FMA ? 1 : 0;
-  const Picks &pk = picks(d->stencil, d->dtype, fma);
-  if (b < 1 || b > pk.maxb)
-    return fail(GBS_ERR_UNSUPPORTED, "no kernel of degree %d built for %s", b, s->name);
-  {
-    if (s->dim == 2) {
-      Geometry2D g = geometry2d(L, b, sl, resident_warps_2d(d->stencil, d->dtype, fma, b));
-      gbs_status st = validate2d(L, g);
-      if (st != GBS_OK) return st;
-      Launch2D a{};
-      a.src = src;
-      a.dst = dst;
-      a.err = err;
-      a.pitch = L.pitch;
-      a.d0 = L.dims[0];
-      a.d1 = L.dims[1];
-      a.shift = L.shift;
-      a.b = b;
-      a.wout = g.wout;
-      a.nstrips = g.nstrips;
-      a.nblocks = g.nblocks;
-      a.sl = g.sl;
-      a.coef = coef;
-      a.div = div;
-      a.eps = eps;
-      a.div_proven = d->dtype == GBS_F32 && div_proven_exact(div);
-      a.stash = stash;
-      a.stash_stride = L.plane;
-      Launch2DFn fn = stash ? pk.l2s[b] : pk.l2[b];
-      if (!fn) return fail(GBS_ERR_UNSUPPORTED, "no 2-D kernel%s for b=%d", stash ? " in stash mode" : "", b);
-      cudaError_t e = fn(a, stream);
-      if (e != cudaSuccess) return cuda_fail(e, "2-D stencil launch");
-    } else {
-      const int v = variant_3d(d, b);
-      if (v < 0) return GBS_ERR_UNSUPPORTED;
-      Geometry3D g = geometry3d(L, b, tile_shape_3d(d->stencil, d->dtype, fma, b, v), sl,
-                                 resident_ctas_3d(d->stencil, d->dtype, fma, b, v));
-      gbs_status st = validate3d(L, g);
-      if (st != GBS_OK) return st;
-      Launch3D a{};
-      a.src = src;
-      a.dst = dst;
-      a.err = err;
-      a.pitch = L.pitch;
-      a.d0 = L.dims[0];
-      a.d1 = L.dims[1];
-      a.d2 = L.dims[2];
-      a.shift = (int)L.shift;
-      a.b = b;
-      a.jout = g.jout;
-      a.wk = g.wk;
-      a.ntk = g.ntk;
-      a.ntj = g.ntj;
-      a.nblocks = g.nblocks;
-      a.sl = g.sl;
-      a.coef = coef;
-      a.div = div;
-      a.div_proven = d->dtype == GBS_F32 && div_proven_exact(div);
-      if (!pk.l3[b][v]) return fail(GBS_ERR_UNSUPPORTED, "no 3-D kernel for b=%d", b);
-      cudaError_t e = pk.l3[b][v](a, stream);
-      if (e != cudaSuccess) return cuda_fail(e, "3-D stencil launch");
-    }
-  }
-  return GBS_OK;
+  BlockPlan plan;
+  gbs_status st = plan_block(d, L, coef, div, eps, sl, b, stash != nullptr, err, &plan);
+  return st == GBS_OK ? launch_plan(plan, src, dst, stash, stream, false) : st;
 }
 }  // namespace gbs
 

@@ -54,9 +54,28 @@ std::vector<int> split_steps(int T, int bt);
 // resident_warps: warps the GPU holds at once for this kernel (0 = unknown)
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident_warps);
 long long resident_warps_2d(int sid, int dtype, int fma, int b);
+// output columns per strip of the 2-D kernels (Pipe2D::WOUT): the window loses
+// b*r columns on the right and b*r rounded up to whole lanes on the left
+inline int wout2d(int rad, int b, int V) {
+  const int left = (b * rad + V - 1) / V * V;
+  return (32 * V - left - b * rad) / V * V;
+}
 gbs_status validate2d(const Layout &L, const Geometry2D &g);
 gbs_status error_word(int **out);
 gbs_status run_loop(const gbs_desc *d, const Layout &L, void *dev_A, cudaStream_t stream, int *err);
+// One kernel launch of b fused steps, planned: everything but its planes.
+struct BlockPlan {
+  int dim;
+  Launch2D a2;
+  Launch2DFn f2;
+  Launch3D a3;
+  Launch3DFn f3;
+};
+// `coef` must outlive the plan
+gbs_status plan_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl, int b,
+                      bool stash, int *err, BlockPlan *out);
+// pdl: the stream's previous operation is a stencil launch (see Launch2D::pdl)
+gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream, bool pdl);
 gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                         int b, const void *src, void *dst, cudaStream_t stream, int *err);
 // launch_block that also stores the states after 1 .. b-1 steps (interior

@@ -56,6 +56,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+// ---- programmatic dependent launch ---------------------------------------------
+// Waits until the kernel this one was started behind has finished and its
+// writes are visible (returns at once in a plain launch). The kernels never
+// trigger their dependents early: CTAs that start while a grid of fewer than
+// one wave still runs crowd onto its idle SMs and stay there (j2d9pt f64
+// 1777x2500: 101 us a step without an early trigger, 175 with one at the
+// kernel's start, 138 with one at its end); the launch itself still overlaps
+// (star2d1r f32 4096^2, degree 4: 7.8 us a step as plain launches, 7.2).
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
@@ -108,6 +118,18 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, unsigned by
           smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+
+// ---- per-thread async copies (16 bytes, L2 only) ------------------------------
+// global -> shared, completed per thread: a thread that waits for its own
+// groups may read what it copied itself, with no barrier.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// waits until at most N of this thread's newest groups are still in flight
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ---- vectors of V elements (16 bytes) ----------------------------------------
@@ -337,6 +359,34 @@ __device__ __forceinline__ float div_by_fast(float x, float d, float y) {
   if (a >= 0x1p-125f && a <= 0x1p+126f) return q1;
   if (x == 0.0f) return __fmul_rn(x, y);
   return __fdiv_rn(x, d);
+}
+
+// The same for V elements at once: one test of the whole vector instead of
+// four branches (with x in the tested range, the quotient is too), and one
+// copy of the rare path, kept out of line so that the row loops stay in the
+// instruction cache.
+__device__ __noinline__ inline float div_rare(float x, float d, float y) { return div_by_fast(x, d, y); }
+template <int V>
+__device__ __forceinline__ void div_by_fast(float (&x)[V], float d, float y) {
+  // |x| in [2^-117, 2^126] for every element: |x/d| in [2^-125, 2^126] for
+  // 1 <= d <= 256 (the proven divisors are 118 and 159)
+  unsigned lo = 0xffffffffu, hi = 0u;
+  float q[V];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    const unsigned a = __float_as_uint(x[e]) & 0x7fffffffu;
+    lo = min(lo, a);
+    hi = max(hi, a);
+    const float q0 = __fmul_rn(x[e], y);
+    const float r = __fmaf_rn(-q0, d, x[e]);
+    q[e] = __fmaf_rn(r, y, q0);
+  }
+  if (lo < 0x05000000u || hi > 0x7e800000u) {  // 2^-117, 2^126
+#pragma unroll
+    for (int e = 0; e < V; ++e) q[e] = x[e] == 0.0f ? __fmul_rn(x[e], y) : div_rare(x[e], d, y);
+  }
+#pragma unroll
+  for (int e = 0; e < V; ++e) x[e] = q[e];
 }
 
 // RN(1/d) for div_by, or 0 when d is outside the range div_by's test covers.

@@ -9,15 +9,18 @@ namespace gbs {
 struct Launch2D {
   const void *src;
   void *dst;
-  int *err;
   long long pitch;
-  int d0, d1, shift, b, wout, nstrips, nblocks, sl;
+  int d0, d1, shift, wout, nstrips, nblocks, sl;
   const double *coef;
   double div, eps;
   bool div_proven;    // the one-correction quotient is exact for every float input
   void *stash;        // not null: level l < b also stores its interior cells to
                       // stash + (l-1)*stash_stride elements (the states between)
   long long stash_stride;
+  // the stream's previous operation is a launch of this family: start this
+  // one while that one drains (programmatic dependent launch; the kernels
+  // wait for it before they touch a grid)
+  bool pdl;
 };
 
 // One launch of the 3-D family (see kernel3d.cuh).
@@ -32,7 +35,26 @@ struct Launch3D {
   const double *coef;
   double div;
   bool div_proven;
+  bool pdl;           // as in Launch2D
 };
+
+// kern<<<grid, block, smem, stream>>>(p), with the programmatic-dependent-launch
+// attribute when pdl is set
+template <class P>
+cudaError_t launch_kernel(void (*kern)(P), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, bool pdl,
+                          const P &p) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
 
 using Launch2DFn = cudaError_t (*)(const Launch2D &, cudaStream_t);
 // resident warps per SM of a 2-D launcher (occupancy), 0 on error

@@ -8,11 +8,16 @@
 //
 // Work decomposition. One WARP is the unit of work; warps never wait on each
 // other. A warp owns a strip of output columns [cs, ce) (wout wide) and a
-// block of output rows [i0, i1) (sl long). It streams level-0 rows
-// i0-b*r .. i1-1+b*r through a per-warp ring of NSTAGE shared-memory row
-// buffers filled by bulk-async (TMA) copies, one 32*V-element window row per
-// copy (V = 16 bytes / element size, 512 bytes per copy). Lane l holds window
-// elements [l*V, l*V+V).
+// block of output rows [i0, i1) (sl long). Lane l holds the V columns
+// [l*V, l*V+V) of the strip's 32*V-column window, one 16-byte vector per row
+// (V = 4 for float, 2 for double).
+//
+// Row pipeline. Level-0 rows i0-b*r .. i1-1+b*r stream through a ring of
+// row buffers in shared memory, filled by 16-byte cp.async copies: every
+// lane copies its own columns and reads back only what it copied, so a row
+// needs no barrier, no vote and no elected lane. Rows are handled in groups
+// of kNph (the unroll of the row loop): one commit and one wait per group,
+// kPrefetch groups in flight ahead of the one being computed.
 //
 // Per fused time level l (1..b) the warp keeps a (2r+1)-row register window.
 // At pipeline step p (level-0 row p arrives) level l produces row p - l*r,
@@ -44,13 +49,10 @@ namespace gbs {
 template <typename T, int NT> struct Params2D {
   const T *src;        // plane read (row 0, element 0 of the padded row)
   T *dst;              // plane written
-  int *err;            // error word (bounded waits)
   long long pitch;     // elements per padded row
   int d0, d1;          // dimsize: rows, columns (interior + 2r)
   int shift;           // column c is stored at element shift + c
-  int b;               // time levels fused in this launch (the kernel's B)
-  int wout;            // output columns per strip (multiple of V)
-  int nstrips, nblocks, sl;
+  int nstrips, nblocks, sl;  // strips of Pipe2D::WOUT columns, stream blocks of sl rows
   T coef[NT];
   T div, rdiv, eps;    // divisor, RN(1/divisor), gradient epsilon
   int divmode;         // 0: no division (folded into coef), 1: checked, 2: proven fast path
@@ -58,14 +60,25 @@ template <typename T, int NT> struct Params2D {
   long long stash_stride;  // stash + (l-1)*stash_stride (the states between)
 };
 
-// y / div as the params ask (see div_by / div_by_fast)
-template <typename T, int NT>
-__device__ __forceinline__ T apply_div(T y, const Params2D<T, NT> &p) {
+// y / div for a lane's elements, as the params ask (see div_by / div_by_fast)
+template <typename T, int V, int NT>
+__device__ __forceinline__ void apply_div(T (&y)[V], const Params2D<T, NT> &p) {
   if constexpr (sizeof(T) == 4) {
-    if (p.divmode == 2) return div_by_fast(y, p.div, p.rdiv);
+    if (p.divmode == 2) {
+      div_by_fast(y, p.div, p.rdiv);
+      return;
+    }
   }
-  if (p.divmode == 0) return y;
-  return div_by(y, p.div, p.rdiv);
+  if (p.divmode == 0) return;
+#pragma unroll 1
+  for (int e = 0; e < V; ++e) {  // one copy of the long checked division
+    T v = y[0];
+#pragma unroll
+    for (int k = 1; k < V; ++k) v = k == e ? y[k] : v;
+    v = div_by(v, p.div, p.rdiv);
+#pragma unroll
+    for (int k = 0; k < V; ++k) y[k] = k == e ? v : y[k];
+  }
 }
 
 // Compile-time facts about a stencil's term list.
@@ -102,96 +115,146 @@ __device__ __forceinline__ void extend_row(T (&ext)[V + 2 * ST::kRad], const T (
 }
 
 
-// One fused time level: the level-(l) row x arrives, the level-(l+1) row q
-// leaves in x. CAREFUL handles halo rows and columns (grid edges);
-// otherwise the caller guarantees that every row and column is interior.
-// Level-0 rows a warp's ring keeps after they arrive: the assoc form carries
-// halo cells of row q (up to b*r rows back) from the ring; the direct form
-// carries them from its register window.
-template <class ST, int B> constexpr int ring_keep2d() { return ST::kAssoc ? B * ST::kRad : 0; }
+// Shape of a warp's row pipeline for (stencil, element type, degree).
+template <class ST, typename T, int B, bool FMA> struct Pipe2D {
+  static constexpr int R = ST::kRad;
+  static constexpr int W = 2 * R + 1;
+  // One 16-byte vector per lane. (Two for double, whose 128-column window
+  // would lose half as large a share of its lanes to the overlap, measured
+  // 3% to 14% slower at degree 1: j2d9pt f64 8192^2 1272 us a step against
+  // 1240, box2d1r 4096^2 326 against 286.)
+  static constexpr int V = 16 / (int)sizeof(T);
+  static constexpr int COLS = 32 * V;
+  static constexpr unsigned ROWB = 512;           // bytes of one ring row
+  // The row loop is unrolled over the window's W positions, which rotates the
+  // window by renaming, where that body stays within about 1300 instructions
+  // (20 KB; it exists once per Care2D). Larger ones slide a window of
+  // W + kNph - 1 rows and move it once per kNph rows, as many as about 800
+  // instructions hold: box2d4r f32 at 4096^2 took 79 us a step unrolled by
+  // three and 69 us by one or two, box2d2r at degree 2 within 3% either way,
+  // star2d3r at degree 3 22 us by four and 20 us by seven. (Instructions of
+  // one row: the sums, a dozen for shuffles and window per level, the copy
+  // and the store.)
+  static constexpr int ROW_INSTR = B * (ST::kTerms * V * (FMA ? 1 : 2) + (ST::kHasDiv && !FMA ? 36 : 0) + 12) + 14;
+  static constexpr bool ROT = sizeof(T) == 8 || W * ROW_INSTR <= 1300;
+  static constexpr int SLIDE = 800 / ROW_INSTR;
+  static constexpr int NPH = ROT ? W : (SLIDE < 1 ? 1 : (SLIDE > W - 1 ? W - 1 : SLIDE));
+  static constexpr int WSLOTS = ROT ? W : W + NPH - 1;
+  // groups in flight ahead of the one being computed: at least 8 rows for
+  // float; 4 for double, whose larger ring would cost resident CTAs
+  static constexpr int PG = ((sizeof(T) == 8 ? 4 : 8) + NPH - 1) / NPH;
+  // level-0 rows kept after they arrive: the assoc form's halo cells take
+  // their fixed values (of rows up to b*r back) from the ring
+  static constexpr int KEEP = ST::kAssoc ? B * R : 0;
+  static constexpr int KG = (KEEP + NPH - 1) / NPH;
+  static constexpr int NROWS = (PG + 1 + KG) * NPH;  // rows of the ring
+  static constexpr unsigned RING = NROWS * ROWB;     // bytes per warp
+  // columns of the window left of the first output column: the overlap b*r
+  // rounded up to whole lanes, so that a lane's vector is stored whole
+  static constexpr int ML = (B * R + V - 1) / V * V;
+  static constexpr int WOUT = (COLS - ML - B * R) / V * V;
+};
 
-// Where an assoc-form level finds the fixed halo values of row q: the warp's
-// ring, which still holds level-0 row q (load index q - pstart). Reading
-// them there costs a shared-memory load instead of a memory round trip in
-// every step of a warp at the grid's edge.
-template <typename T, int NSTAGE> struct CarryRing {
-  const T *ring;        // the warp's ring + lane * V
-  unsigned base;        // the item's first load index on the ring
-  int pstart;           // row of load index 0
-  int nrows;            // rows loaded by the item
-  __device__ __forceinline__ const T *row(int q) const {
-    const int n = q - pstart;
-    return (n >= 0 && n < nrows) ? ring + (size_t)((base + (unsigned)n) % NSTAGE) * (32 * (16 / sizeof(T)))
-                                 : nullptr;
+// the lane's elements of a ring row (p: the row + lane * 16)
+template <class PP, typename T>
+__device__ __forceinline__ void ld_ring(T (&x)[PP::V], const unsigned char *p) {
+  ld_vec<T, PP::V>(x, reinterpret_cast<const T *>(p));
+}
+
+// window slot of logical position j (0 = oldest row) in phase ph
+template <class PP> __host__ __device__ constexpr int slot2d(int ph, int j) {
+  return PP::ROT ? (ph + 1 + j) % PP::W : ph + j;
+}
+
+// Halo values for the assoc form: the level-0 row q of the lane, in the ring
+// for b*r rows after it arrived. Read unconditionally, ahead of the sums that
+// hide its latency; for a row that was never loaded the ring's stale contents
+// reach only rows and columns that no output needs.
+template <class PP> struct CarryRing {
+  const unsigned char *ring;  // the warp's ring + lane * 16
+  int cur, cur_row;           // ring row index and grid row of the group's first row
+  template <typename T> __device__ __forceinline__ void row(T (&x)[PP::V], int q) const {
+    int s = cur + (q - cur_row);
+    if (s < 0) s += PP::NROWS;
+    ld_ring<PP>(x, ring + (unsigned)s * PP::ROWB);
   }
 };
 
-template <class ST, typename T, bool FMA, bool UNR, bool CAREFUL, int PH, int V, int NSTAGE>
-__device__ __forceinline__ void level2d(T (&win)[2 * ST::kRad + 1][V], T (&x)[V], int q, bool edge,
-                                        int col0, const CarryRing<T, NSTAGE> &carry,
+// What a group of rows may meet. Three copies of the row code: all warps of a
+// launch start together, so the strips at the grid's left and right edge set
+// its end if their rows cost much more than the others' (with the halo-row
+// tests in every edge row, branches and late ring reads, box2d1r f32 at
+// 4096^2, degree 4, took 13.8 us a step; 10.0 now).
+enum Care2D : int {
+  kInterior = 0,  // interior rows and columns only
+  kColumns = 1,   // halo columns (a strip at the grid's left or right edge), interior rows
+  kAll = 2        // halo rows as well
+};
+
+// One fused time level: the level-(l) row x arrives, the level-(l+1) row q
+// leaves in x.
+// The sums of the few overlap rows that no output needs are computed all the
+// same: a test per row and level costs more than it saves, on the FP64 pipe
+// too (star2d1r f64 16384^2 2755 us a step with it, 2444 without).
+template <class ST, class PP, typename T, bool FMA, int CARE, int PH>
+__device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&x)[PP::V], int q,
+                                        const bool (&fixed)[PP::V], const CarryRing<PP> &carry,
                                         const Params2D<T, ST::kTerms> &p) {
   constexpr int R = ST::kRad;
-  constexpr int W = 2 * R + 1;
+  constexpr int V = PP::V;
   using A = Arith<T>;
   T y[V];
   bool halo_row = false;
-  if constexpr (CAREFUL) halo_row = (q < R) || (q >= p.d0 - R);
+  if constexpr (CARE == kAll) halo_row = (q < R) || (q >= p.d0 - R);
   if constexpr (!ST::kAssoc) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) win[wslot<UNR, W>(PH, 2 * R)][e] = x[e];
-    constexpr int cslot = wslot<UNR, W>(PH, R);
-    if (CAREFUL && halo_row) {
-#pragma unroll
-      for (int e = 0; e < V; ++e) y[e] = win[cslot][e];
-    } else {
-      if constexpr (ST::kKind == KIND_GRADIENT) {
-        T ext[V + 2 * R];
-        extend_row<ST, V, 0>(ext, win[cslot]);
-        static_for<V>([&](auto EI) {
-          constexpr int e = decltype(EI)::value;
-          T nb[ST::kTerms];
-          static_for<ST::kTerms>([&](auto TI) {
-            constexpr int t = decltype(TI)::value;
-            constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-            if constexpr (di == 0) nb[t] = ext[R + e + dj];
-            else nb[t] = win[wslot<UNR, W>(PH, R + di)][e];
-          });
-          y[e] = gradient_update<T, ST::kTerms, FMA>(win[cslot][e], nb, p.eps, p.coef[0]);
-        });
-      } else {
-        // the direct form serves stencils whose off-centre rows are read at
-        // the centre column only (stars, star2d4r): one extended row
-        T ext[V + 2 * R];
-        extend_row<ST, V, 0>(ext, win[cslot]);
-        static_for<ST::kTerms>([&](auto TI) {
+    for (int e = 0; e < V; ++e) win[slot2d<PP>(PH, 2 * R)][e] = x[e];
+    constexpr int cslot = slot2d<PP>(PH, R);
+    if constexpr (ST::kKind == KIND_GRADIENT) {
+      T ext[V + 2 * R];
+      extend_row<ST, V, 0>(ext, win[cslot]);
+      static_for<V>([&](auto EI) GBS_INL {
+        constexpr int e = decltype(EI)::value;
+        T nb[ST::kTerms];
+        static_for<ST::kTerms>([&](auto TI) GBS_INL {
           constexpr int t = decltype(TI)::value;
           constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-          static_assert(di == 0 || dj == 0, "direct 2-D form expects off-centre rows at dj == 0");
-          constexpr int slot = wslot<UNR, W>(PH, R + di);
-          static_for<V>([&](auto EI) {
-            constexpr int e = decltype(EI)::value;
-            T a;
-            if constexpr (dj == 0) a = win[slot][e];
-            else a = ext[R + e + dj];
-            if constexpr (t == 0) y[e] = A::mul(p.coef[t], a);
-            else y[e] = term_next<T, FMA>(y[e], p.coef[t], a);
-          });
+          if constexpr (di == 0) nb[t] = ext[R + e + dj];
+          else nb[t] = win[slot2d<PP>(PH, R + di)][e];
         });
-        if constexpr (ST::kHasDiv && !FMA) {  // FMA mode: folded into the coefficients
+        y[e] = gradient_update<T, ST::kTerms, FMA>(win[cslot][e], nb, p.eps, p.coef[0]);
+      });
+    } else {
+      // the direct form serves stencils whose off-centre rows are read at
+      // the centre column only (stars, star2d4r): one extended row
+      T ext[V + 2 * R];
+      extend_row<ST, V, 0>(ext, win[cslot]);
+      static_for<ST::kTerms>([&](auto TI) GBS_INL {
+        constexpr int t = decltype(TI)::value;
+        constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
+        static_assert(di == 0 || dj == 0, "direct 2-D form expects off-centre rows at dj == 0");
+        constexpr int slot = slot2d<PP>(PH, R + di);
+        static_for<V>([&](auto EI) GBS_INL {
+          constexpr int e = decltype(EI)::value;
+          T a;
+          if constexpr (dj == 0) a = win[slot][e];
+          else a = ext[R + e + dj];
+          if constexpr (t == 0) y[e] = A::mul(p.coef[t], a);
+          else y[e] = term_next<T, FMA>(y[e], p.coef[t], a);
+        });
+      });
+      if constexpr (ST::kHasDiv && !FMA) apply_div(y, p);  // FMA mode: folded into the coefficients
+    }
+    if constexpr (CARE != kInterior) {
 #pragma unroll
-          for (int e = 0; e < V; ++e) y[e] = apply_div(y[e], p);
-        }
-      }
-      if (CAREFUL && edge) {
-#pragma unroll
-        for (int e = 0; e < V; ++e)
-          if (col0 + e < R || col0 + e >= p.d1 - R) y[e] = win[cslot][e];
-      }
+      for (int e = 0; e < V; ++e) y[e] = (halo_row || fixed[e]) ? win[cslot][e] : y[e];
     }
   } else {
     // assoc: the arriving row m = q + R adds its terms to outputs q..q+2R
+    T cv[V];
+    if constexpr (CARE != kInterior) carry.row(cv, q);
     T ext[V + 2 * R];
-    static_for<V + 2 * R>([&](auto XI) {
+    static_for<V + 2 * R>([&](auto XI) GBS_INL {
       constexpr int xx = decltype(XI)::value - R;
       constexpr bool any = [] {
         for (int di = -R; di <= R; ++di)
@@ -200,42 +263,31 @@ __device__ __forceinline__ void level2d(T (&win)[2 * ST::kRad + 1][V], T (&x)[V]
       }();
       if constexpr (any) ext[R + xx] = row_elem<V, xx>(x);
     });
-    static_for<ST::kTerms>([&](auto TI) {
-      constexpr int t = decltype(TI)::value;
-      constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-      constexpr int slot = wslot<UNR, W>(PH, R - di);
-      static_for<V>([&](auto EI) {
-        constexpr int e = decltype(EI)::value;
-        const T a = ext[R + e + dj];
-        if constexpr (t == 0) win[slot][e] = A::mul(p.coef[t], a);
-        else win[slot][e] = term_next<T, FMA>(win[slot][e], p.coef[t], a);
+    // term by term in source order, one row offset after the other
+    static_for<PP::W>([&](auto DI) GBS_INL {
+      constexpr int di = decltype(DI)::value - R;
+      static_for<ST::kTerms>([&](auto TI) GBS_INL {
+        constexpr int t = decltype(TI)::value;
+        if constexpr (ST::kOff[t][0] == di) {
+          constexpr int dj = ST::kOff[t][1];
+          constexpr int slot = slot2d<PP>(PH, R - di);
+          static_for<V>([&](auto EI) GBS_INL {
+            constexpr int e = decltype(EI)::value;
+            const T a = ext[R + e + dj];
+            if constexpr (t == 0) win[slot][e] = A::mul(p.coef[t], a);
+            else win[slot][e] = term_next<T, FMA>(win[slot][e], p.coef[t], a);
+          });
+        }
       });
     });
-    constexpr int oslot = wslot<UNR, W>(PH, 0);
+    constexpr int oslot = slot2d<PP>(PH, 0);
 #pragma unroll
     for (int e = 0; e < V; ++e) y[e] = win[oslot][e];
-    if constexpr (ST::kHasDiv && !FMA) {  // FMA mode: folded into the coefficients
+    if constexpr (ST::kHasDiv && !FMA) apply_div(y, p);  // FMA mode: folded into the coefficients
+    if constexpr (CARE != kInterior) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) y[e] = apply_div(y[e], p);
+      for (int e = 0; e < V; ++e) y[e] = (halo_row || fixed[e]) ? cv[e] : y[e];
     }
-    if constexpr (CAREFUL) {
-      if (halo_row || edge) {
-        const T *c = (q >= 0 && q < p.d0) ? carry.row(q) : nullptr;
-        if (c) {
-          T cv[V];
-          ld_vec<T, V>(cv, c);
-#pragma unroll
-          for (int e = 0; e < V; ++e)
-            if (halo_row || col0 + e < R || col0 + e >= p.d1 - R) y[e] = cv[e];
-        }
-      }
-    }
-  }
-  if constexpr (!UNR) {
-#pragma unroll
-    for (int j = 0; j < 2 * R; ++j)
-#pragma unroll
-      for (int e = 0; e < V; ++e) win[j][e] = win[j + 1][e];
   }
 #pragma unroll
   for (int e = 0; e < V; ++e) x[e] = y[e];
@@ -243,235 +295,198 @@ __device__ __forceinline__ void level2d(T (&win)[2 * ST::kRad + 1][V], T (&x)[V]
 
 // One work item of a warp: output columns [cs, ce) of strip `strip` and
 // output rows [i0, i1) of stream block `blk`, advanced by B levels from p.src
-// into p.dst. `ring`/`bars` are the warp's NSTAGE row buffers and their
-// mbarriers (initialised by the caller); `load_base` counts the copies this
-// warp has issued on them so far, so that items can follow each other on the
-// same barriers. Returns false when a bounded wait gave up (p.err is set and
-// the copies in flight have been drained).
+// into p.dst. `ring` is the warp's Pipe2D::RING bytes of shared memory
+// (16-byte aligned), owned by this warp.
 // STASH: the intermediate levels also store their rows (the states after 1
 // .. B-1 steps) in the item's output rows and columns, where every level is
 // valid, to p.stash; a separate instantiation, so that the plain kernels
 // carry none of it.
-template <class ST, typename T, int B, bool FMA, int NSTAGE, bool STASH = false>
-__device__ __forceinline__ bool warp_item2d(const Params2D<T, ST::kTerms> &p, int strip, int blk, T *ring,
-                                            uint64_t *bars, unsigned &load_base) {
-  constexpr int V = 16 / sizeof(T);
-  constexpr int R = ST::kRad;
-  constexpr int W = 2 * R + 1;
-  constexpr bool UNR = (R <= 2);
-  constexpr int NPH = UNR ? W : 1;
-  constexpr int ROW = 32 * V;
-  constexpr unsigned ROW_BYTES = ROW * sizeof(T);
+//
+// What bounds it and what it measured: see stencil2d_kernel.
+template <class ST, typename T, int B, bool FMA, bool STASH = false>
+__device__ __forceinline__ void warp_item2d(const Params2D<T, ST::kTerms> &p, int strip, int blk,
+                                            unsigned char *ring) {
+  using PP = Pipe2D<ST, T, B, FMA>;
+  constexpr int V = PP::V, R = PP::R, NPH = PP::NPH, PG = PP::PG;
   const int lane = threadIdx.x & 31;
 
-  // ---- columns (column space c; offset space c + shift) ----
-  const int cs = R + strip * p.wout;
-  const int ce = min(cs + p.wout, p.d1 - R);
-  const int need_lo = max(0, cs - B * R);
-  const int ws = ((need_lo + p.shift) / V) * V;
-  const int col0 = ws - p.shift + lane * V;  // column of this lane's element 0
-  const bool edge = (ws - p.shift < R) || (ws - p.shift + ROW > p.d1 - R);
+  // ---- columns (column space c; element space c + shift) ----
+  const int cs = R + strip * PP::WOUT;
+  const int ce = min(cs + PP::WOUT, p.d1 - R);
+  const int ws = cs + p.shift - PP::ML;          // element of the window's column 0 (may be negative)
+  const int el = ws + lane * V;                  // this lane's first element
+  const int col0 = el - p.shift;                 // and its column
+  const bool edge = (ws - p.shift < R) || (ws - p.shift + PP::COLS > p.d1 - R);
   const bool store_all = (col0 >= cs && col0 + V <= ce);
+  bool fixed[V];                                 // halo columns (and columns off the grid)
+#pragma unroll
+  for (int e = 0; e < V; ++e) fixed[e] = (col0 + e < R || col0 + e >= p.d1 - R);
 
   // ---- rows ----
   const int i0 = R + blk * p.sl;
   const int i1 = min(i0 + p.sl, p.d0 - R);
   const int pstart = max(0, i0 - B * R);
-  const int pend = min(p.d0, i1 + B * R);  // rows loaded: [pstart, pend)
-  const int plast = i1 - 1 + B * R;        // last pipeline step
-  const int nload = pend - pstart;
+  const int pend = min(p.d0, i1 + B * R);        // rows loaded: [pstart, pend)
+  const int ng = (i1 + B * R - pstart + NPH - 1) / NPH;
+  // rows [fast_lo, fast_hi): every level's row is interior (or not needed)
+  const int fast_lo = i0 >= B * R ? pstart : (B + 1) * R;
+  const int fast_hi = i1 + B * R <= p.d0 ? 0x7fffffff : p.d0;
 
-  const T *src_win = p.src + ws;
-  T *dst_lane = p.dst + ws + lane * V;
-  const long long pitch = p.pitch;
-  const unsigned base = load_base;
-  constexpr int KEEP = ring_keep2d<ST, B>();
-  static_assert(KEEP + 2 <= NSTAGE, "the ring must keep b*r rows and still prefetch");
-  const CarryRing<T, NSTAGE> carry{ring + lane * V, base, pstart, nload};
-
-  if (lane == 0) {
-#pragma unroll 1
-    for (int n = 0; n < NSTAGE && n < nload; ++n) {
-      const unsigned s = (base + n) % NSTAGE;
-      mbar_arrive_expect_tx(&bars[s], ROW_BYTES);
-      bulk_g2s(ring + s * ROW, src_win + (long long)(pstart + n) * p.pitch, ROW_BYTES, &bars[s]);
+  // ---- copies: lane-private, one vector per row ----
+  unsigned char *my = ring + lane * 16;
+  const uint32_t my_s = smem_u32(my);
+  const bool in_row = el >= 0 && el + V <= p.pitch;
+  const T *ld = p.src + (long long)pstart * p.pitch + el;
+  int ld_left = pend - pstart;                   // rows not yet requested
+  unsigned wr = 0;                               // byte offset of the next group's first row
+  auto request_group = [&]() GBS_INL {
+#pragma unroll
+    for (int ph = 0; ph < NPH; ++ph) {
+      if (in_row && ph < ld_left) cp_async16(my_s + wr + (unsigned)ph * PP::ROWB, ld);
+      ld += p.pitch;
     }
-  }
-  __syncwarp();
+    cp_async_commit();
+    ld_left -= NPH;
+    wr = wr + NPH * PP::ROWB == PP::RING ? 0u : wr + NPH * PP::ROWB;
+  };
+#pragma unroll 1
+  for (int g = 0; g < PG; ++g) request_group();
 
-  T win[B][W][V];
+  T win[B][PP::WSLOTS][V];
 #pragma unroll
   for (int l = 0; l < B; ++l)
 #pragma unroll
-    for (int w = 0; w < W; ++w)
+    for (int w = 0; w < PP::WSLOTS; ++w)
 #pragma unroll
       for (int e = 0; e < V; ++e) win[l][w][e] = T(0);
 
-  int consumed = 0;  // loads consumed so far (for the drain on timeout)
-  bool ok = true;
+  unsigned rd = 0;                               // byte offset of the group being computed
+  T *st = p.dst + (long long)(pstart - B * R) * p.pitch + el;  // row the last level stores in the first step
+  T *ss = STASH ? p.stash + (long long)pstart * p.pitch + el : nullptr;
+  const unsigned nout = (unsigned)(i1 - i0);
+  int pb = pstart;                               // row of the group's phase 0
 
-  // One pipeline step at row pp with phase PH. CAREFUL steps handle the
-  // stream ends, halo rows and edge columns; the others assume none occur.
-  auto step = [&](auto PHI, auto CAREI, int pp) GBS_INL {
-    constexpr int ph = decltype(PHI)::value;
-    constexpr bool careful = decltype(CAREI)::value;
-    T x[V];
-    if (!careful || pp < pend) {
-      const int n = pp - pstart;
-      const unsigned gn = base + n;
-      const unsigned s = gn % NSTAGE;
-      // every lane waits; the decision to give up is warp-uniform
-      const bool got = mbar_wait(&bars[s], (gn / NSTAGE) & 1u, nullptr, 0);
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) atomicOr(p.err, ERR_WAIT_TIMEOUT);
-        ok = false;
-        return;
-      }
-      ld_vec<T, V>(x, ring + s * ROW + lane * V);
-      consumed = n + 1;
-    } else {
+  // rows pb .. pb+NPH-1, with what CAREI (Care2D) says they meet. Rows past the item's last are computed from
+  // whatever the ring holds and never stored.
+  auto rows = [&](auto CAREI) GBS_INL {
+    constexpr int care = decltype(CAREI)::value;
+    const CarryRing<PP> carry{my, (int)(rd / PP::ROWB), pb};
+    static_for<NPH>([&](auto PHI) GBS_INL {
+      constexpr int ph = decltype(PHI)::value;
+      const int pp = pb + ph;
+      T x[V];
+      ld_ring<PP>(x, my + rd + (unsigned)ph * PP::ROWB);
+      static_for<B>([&](auto LI) GBS_INL {
+        constexpr int l = decltype(LI)::value;
+        level2d<ST, PP, T, FMA, care, ph>(win[l], x, pp - (l + 1) * R, fixed, carry, p);
+        if constexpr (STASH && l + 1 < B) {
+          const unsigned ql = (unsigned)(pp - (l + 1) * R - i0);
+          if (ql < nout) {
+            T *d = ss + (long long)l * p.stash_stride - (long long)((l + 1) * R) * p.pitch;
+            if (store_all) {
+              st_vec_global<T, V>(d, x);
+            } else if constexpr (care != kInterior) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) x[e] = T(0);
-    }
-    static_for<B>([&](auto LI) {
-      constexpr int l = decltype(LI)::value;
-      level2d<ST, T, FMA, UNR, careful, ph, V, NSTAGE>(win[l], x, pp - (l + 1) * R, edge, col0, carry, p);
-      if constexpr (STASH && l + 1 < B) {
-        const int ql = pp - (l + 1) * R;
-        if (ql >= i0 && ql < i1) {
-          T *d = p.stash + (long long)l * p.stash_stride + ws + lane * V + (long long)ql * pitch;
-          if (store_all) {
-            st_vec_global<T, V>(d, x);
-          } else {
-#pragma unroll
-            for (int e = 0; e < V; ++e)
-              if (col0 + e >= cs && col0 + e < ce) st_global(d + e, x[e]);
+              for (int e = 0; e < V; ++e)
+                if (col0 + e >= cs && col0 + e < ce) st_global(d + e, x[e]);
+            }
           }
         }
-      }
-    });
-    const int q = pp - B * R;
-    if (q >= i0 && q < i1) {
-      T *d = dst_lane + (long long)q * pitch;
-      if (store_all) {
-        st_vec_global<T, V>(d, x);
-      } else {
-#pragma unroll
-        for (int e = 0; e < V; ++e)
-          if (col0 + e >= cs && col0 + e < ce) st_global(d + e, x[e]);
-      }
-    }
-    // the row KEEP steps back is no longer needed: refill its stage
-    const int nf = pp - pstart - KEEP;
-    if (nf >= 0 && nf + NSTAGE < nload) {
-      __syncwarp();
-      if (lane == 0) {
-        const unsigned sf = (base + nf) % NSTAGE;
-        mbar_arrive_expect_tx(&bars[sf], ROW_BYTES);
-        bulk_g2s(ring + sf * ROW, src_win + (long long)(pstart + nf + NSTAGE) * pitch, ROW_BYTES, &bars[sf]);
-      }
-    }
-  };
-
-  // steps [lo, hi) in whole groups of NPH phases, starting at a group boundary
-  auto run = [&](int lo, int hi, auto CAREI) GBS_INL {
-#pragma unroll 1
-    for (int pb = lo; pb < hi && ok; pb += NPH) {
-      static_for<NPH>([&](auto PHI) {
-        const int pp = pb + decltype(PHI)::value;
-        if (!ok || (decltype(CAREI)::value && pp >= hi)) return;
-        step(PHI, CAREI, pp);
       });
+      if ((unsigned)(pp - B * R - i0) < nout) {
+        if (store_all) {
+          st_vec_global<T, V>(st, x);
+        } else if constexpr (care != kInterior) {
+          // outside the edge strips a lane is stored whole or not at all
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            if (col0 + e >= cs && col0 + e < ce) st_global(st + e, x[e]);
+        }
+      }
+      st += p.pitch;
+      if constexpr (STASH) ss += p.pitch;
+    });
+    if constexpr (!PP::ROT) {
+#pragma unroll
+      for (int l = 0; l < B; ++l)
+#pragma unroll
+        for (int j = 0; j < 2 * R; ++j)
+#pragma unroll
+          for (int e = 0; e < V; ++e) win[l][j][e] = win[l][j + NPH][e];
     }
   };
-  const int steps = plast + 1 - pstart;
-  if (edge) {
-    run(pstart, plast + 1, IC<1>());
-  } else {
-    // rows whose levels all lie in the interior and that are loaded
-    const int mid_lo = max(pstart, (B + 1) * R);
-    const int mid_hi = min(plast + 1, p.d0);
-    int a = pstart + (mid_lo - pstart + NPH - 1) / NPH * NPH;
-    int z = pstart + max(0, mid_hi - pstart) / NPH * NPH;
-    if (a > z) a = z = pstart + steps;  // no interior stretch: all careful
-    run(pstart, min(a, plast + 1), IC<1>());
-    if (a < z) run(a, z, IC<0>());
-    if (z < plast + 1) run(z, plast + 1, IC<1>());
-  }
 
-  if (!ok) {
-    if (lane == 0) {
-      // Timed out: wait (bounded) for the copies still in flight into this
-      // warp's ring before the CTA may exit and release its shared memory.
-      const int issued = min(nload, max(NSTAGE, consumed + NSTAGE - KEEP));
-      for (int n = consumed; n < issued; ++n) {
-        const unsigned gn = base + n;
-        if (!mbar_wait(&bars[gn % NSTAGE], (gn / NSTAGE) & 1u, p.err, ERR_DRAIN_TIMEOUT)) break;
-      }
-    }
-    return false;
+#pragma unroll 1
+  for (int g = 0; g < ng; ++g) {
+    request_group();           // group g + PG, into the slot freed by the group before the kept ones
+    cp_async_wait<PG>();       // group g has landed (this lane's own copies)
+    if (pb < fast_lo || pb + NPH > fast_hi) rows(IC<kAll>());
+    else if (edge) rows(IC<kColumns>());
+    else rows(IC<kInterior>());
+    pb += NPH;
+    rd = rd + NPH * PP::ROWB == PP::RING ? 0u : rd + NPH * PP::ROWB;
   }
-  load_base = base + nload;
-  return true;
+  cp_async_wait<0>();          // nothing in flight into the ring when the next item starts
 }
 
-// The warp's ring and barriers inside the CTA's dynamic shared memory.
-template <typename T, int WPC, int NSTAGE>
-__device__ __forceinline__ void warp_ring2d(unsigned char *smem_raw, T *&ring, uint64_t *&bars) {
-  constexpr int ROW = 32 * (16 / sizeof(T));
-  const int wid = threadIdx.x >> 5;
-  ring = reinterpret_cast<T *>(smem_raw) + (size_t)wid * NSTAGE * ROW;
-  bars = reinterpret_cast<uint64_t *>(smem_raw + (size_t)WPC * NSTAGE * ROW * sizeof(T)) + wid * NSTAGE;
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int s = 0; s < NSTAGE; ++s) mbar_init(&bars[s], 1);
-    fence_mbar_init();
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  __syncwarp();
+constexpr int kWpc2D = kWarpsPerCta2D;
+
+template <class ST, typename T, int B, bool FMA> constexpr size_t smem_bytes2d() {
+  return (size_t)kWpc2D * Pipe2D<ST, T, B, FMA>::RING;
 }
 
-template <class ST, typename T, int B, bool FMA, int WPC, int NSTAGE, bool STASH = false>
-__global__ void __launch_bounds__(WPC * 32, gbs_min_ctas(WPC * 32))
+// Bound: instruction issue at degree 2 and above for float (HBM at degree 1),
+// the FP64 pipe for double. A row of star2d1r at degree 4 takes 122 warp
+// instructions for its 80 multiplies and FMAs; with one bulk copy per row,
+// its mbarrier wait, vote and elected refill it took 191. Measured (GB300,
+// time per step at the tuned degree, before -> after): star2d1r f32 4096^2
+// 13.2 us (degree 4) -> 6.5 (7); j2d5pt f32 16384^2 125 -> 79; box2d2r f32
+// 3001x2217 24.5 -> 13.1; j2d9pt f64 1777x2500 132 (2) -> 85 (1);
+// j2d9pt-gol f32 1500^2, exact mode, 12.8 -> 9.9.
+template <class ST, typename T, int B, bool FMA, bool STASH = false>
+__global__ void __launch_bounds__(kWpc2D * 32, gbs_min_ctas(kWpc2D * 32))
     stencil2d_kernel(const __grid_constant__ Params2D<T, ST::kTerms> p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const long long gw = (long long)blockIdx.x * WPC + (threadIdx.x >> 5);
+  const int w = threadIdx.x >> 5;
+  const long long gw = (long long)blockIdx.x * kWpc2D + w;
+  wait_for_previous();
   if (gw >= (long long)p.nstrips * p.nblocks) return;
-  T *ring;
-  uint64_t *bars;
-  warp_ring2d<T, WPC, NSTAGE>(smem_raw, ring, bars);
-  unsigned load_base = 0;
-  warp_item2d<ST, T, B, FMA, NSTAGE, STASH>(p, (int)(gw % p.nstrips), (int)(gw / p.nstrips), ring, bars,
-                                            load_base);
+  warp_item2d<ST, T, B, FMA, STASH>(p, (int)(gw % p.nstrips), (int)(gw / p.nstrips),
+                                    smem_raw + (size_t)w * Pipe2D<ST, T, B, FMA>::RING);
 }
 
-constexpr int kWpc2D = kWarpsPerCta2D, kStages2D = 16;
+// opts the kernel in to its shared memory (above 48 KB the default refuses the launch)
+template <class K> cudaError_t allow_smem2d(K kern, size_t smem) {
+  if (smem <= 48 * 1024) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
 
 template <class ST, typename T, int B, bool FMA>
 int occupancy2d() {
-  constexpr int V = 16 / sizeof(T);
-  const size_t smem = (size_t)kWpc2D * kStages2D * (32 * V * sizeof(T) + sizeof(uint64_t));
+  constexpr size_t smem = smem_bytes2d<ST, T, B, FMA>();
+  auto kern = stencil2d_kernel<ST, T, B, FMA>;
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, stencil2d_kernel<ST, T, B, FMA, kWpc2D, kStages2D>,
-                                                    kWpc2D * 32, smem) != cudaSuccess)
+  if (allow_smem2d(kern, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kWpc2D * 32, smem) != cudaSuccess)
     return 0;
   return nb * kWpc2D;
 }
 
 template <class ST, typename T, int B, bool FMA, bool STASH = false>
 cudaError_t launch2d(const Launch2D &a, cudaStream_t stream) {
-  constexpr int WPC = kWpc2D, NSTAGE = kStages2D;
-  constexpr int V = 16 / sizeof(T);
+  constexpr size_t smem = smem_bytes2d<ST, T, B, FMA>();
+  auto kern = stencil2d_kernel<ST, T, B, FMA, STASH>;
+  if (STASH != (a.stash != nullptr) || a.wout != Pipe2D<ST, T, B, FMA>::WOUT) return cudaErrorInvalidValue;
+  if (const cudaError_t e = allow_smem2d(kern, smem); e != cudaSuccess) return e;
   Params2D<T, ST::kTerms> p;
   p.src = static_cast<const T *>(a.src);
   p.dst = static_cast<T *>(a.dst);
-  p.err = a.err;
   p.pitch = a.pitch;
   p.d0 = a.d0;
   p.d1 = a.d1;
   p.shift = a.shift;
-  p.b = a.b;
-  p.wout = a.wout;
   p.nstrips = a.nstrips;
   p.nblocks = a.nblocks;
   p.sl = a.sl;
@@ -485,12 +500,9 @@ cudaError_t launch2d(const Launch2D &a, cudaStream_t stream) {
   p.eps = (T)a.eps;
   p.stash = static_cast<T *>(a.stash);
   p.stash_stride = a.stash_stride;
-  if (STASH != (a.stash != nullptr)) return cudaErrorInvalidValue;
-  const size_t smem = (size_t)WPC * NSTAGE * (32 * V * sizeof(T) + sizeof(uint64_t));
   const long long warps = (long long)a.nstrips * a.nblocks;
-  const long long grid = (warps + WPC - 1) / WPC;
-  stencil2d_kernel<ST, T, B, FMA, WPC, NSTAGE, STASH><<<(unsigned)grid, WPC * 32, smem, stream>>>(p);
-  return cudaGetLastError();
+  const long long grid = (warps + kWpc2D - 1) / kWpc2D;
+  return launch_kernel(kern, (unsigned)grid, kWpc2D * 32, smem, stream, a.pdl, p);
 }
 
 }  // namespace gbs

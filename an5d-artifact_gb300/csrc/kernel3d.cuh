@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(TJ * 32, gbs_min_ctas(TJ * 32))
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
+  wait_for_previous();
 
   auto issue = [&](int plane) GBS_INL {  // lane 0 of every warp: this warp's row of `plane`
     const int n = plane - pstart;
@@ -535,7 +536,7 @@ cudaError_t launch3d(const Launch3D &a, cudaStream_t stream) {
     p.nblocks = a.nblocks;
     p.sl = a.sl;
     for (int t = 0; t < ST::kTerms; ++t) p.coef[t] = fold ? (T)(a.coef[t] / a.div) : (T)a.coef[t];
-    kern<<<(unsigned)grid, NT, smem, stream>>>(p);
+    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, a.pdl, p);
   } else {
     Params3D<T, ST::kTerms> p;
     p.src = static_cast<const T *>(a.src);
@@ -556,9 +557,8 @@ cudaError_t launch3d(const Launch3D &a, cudaStream_t stream) {
     p.divmode = !ST::kHasDiv || fold ? 0 : (a.div_proven ? 2 : 1);
     p.div = (T)a.div;
     p.rdiv = div_reciprocal<T>(a.div);
-    kern<<<(unsigned)grid, NT, smem, stream>>>(p);
+    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, a.pdl, p);
   }
-  return cudaGetLastError();
 }
 
 template <class ST, typename T, int B, bool FMA, int NW = kNw3D>
