@@ -20,9 +20,8 @@
 //    partial buffer (no atomics; summed in double at the end).
 // gradient2d, u_{t+1} = u + c q, q = (eps + s)^{-1/2}, s = sum_n (u - u_{x+n})^2:
 //    the linearised update, dF(x)/du(x) = 1 - c q^3 sum_n d_n(x),
-//    dF(x)/du(x+n) = c q^3 d_n(x), dF(x)/dc = q(x), evaluated on u_t: a
-//    pre-pass stores q and sum_n d_n per cell, a gather kernel applies the
-//    transposed Jacobian.
+//    dF(x)/du(x+n) = c q^3 d_n(x), dF(x)/dc = q(x), evaluated on u_t, whose
+//    transpose one streaming pass applies.
 //
 // Checkpointing: gbs_adjoint_forward advances the grid and saves u_t every
 // C steps into the caller's workspace. When the states are needed,
@@ -444,97 +443,199 @@ __global__ void __launch_bounds__(kAdjThreads) adj2d_kernel(const __grid_constan
   }
 }
 
-// gradient2d pre-pass: for interior x, q(x) = (eps + s(x))^{-1/2} and
-// sd(x) = sum_n d_n(x), d_n = u(x) - u(x + n), from u_t (s formed as the
-// forward step forms it)
-template <class ST, typename T>
-__global__ void __launch_bounds__(kAdjThreads) grad_pre_kernel(const __grid_constant__ AdjGeom g, const T *u, T *qp,
-                                                               T *sdp, T eps) {
-  const long long cidx = (long long)blockIdx.x * kAdjThreads + threadIdx.x;
-  if (cidx >= g.cells) return;
-  const int i = (int)(cidx / g.d1), j = (int)(cidx - (long long)(cidx / g.d1) * g.d1);
-  const int R = g.rad;
-  if (!(i >= R && i < g.d0 - R && j >= R && j < g.d1 - R)) return;
-  using A = Arith<T>;
-  const long long o = cell_off(g, i, j, 0);
-  const T ux = u[o];
-  T s = eps;
-  double sd = 0.0;
-  static_for<ST::kTerms>([&](auto TI) {
-    constexpr int t = decltype(TI)::value;
-    const T d = A::sub(ux, u[cell_off(g, i + ST::kOff[t][0], j + ST::kOff[t][1], 0)]);
-    s = A::add(s, A::mul(d, d));
-    sd += (double)d;
-  });
-  // Newton-Raphson for 1/sqrt(s) from a single-precision estimate (two
-  // steps: relative error 2^-22 -> 2^-44 -> double precision)
-  const double sv = (double)s;
-  double y;
-  if (sv >= 1e-30 && sv <= 1e30) {
-    y = (double)rsqrtf((float)s);
-    double h = fma(-sv * y, y, 1.0);
-    y = fma(0.5 * y, h, y);
-    h = fma(-sv * y, y, 1.0);
-    y = fma(0.5 * y, h, y);
-  } else {
-    y = 1.0 / sqrt(sv);
-  }
-  qp[o] = (T)y;
-  sdp[o] = (T)sd;
-}
+// gradient2d adjoint step, one pass over u_t and lam_{t+1}:
+//   lam_t(y) = lam(y) + sum_x (w(x) + w(y)) (u(x) - u(y)),  w = num q^3 lam,
+// over y's four neighbours x, w = 0 on the halo (the transposed linearised
+// Jacobian: -w(y) sum_n d_n(y) and the neighbours' c q^3 d_n share their
+// differences). A term belongs to the edge between two cells and enters both
+// with opposite sign, so each edge's difference, square and flux is formed
+// once. At a halo cell the same sum is the increment of its gradient.
+//
+// A warp owns a strip of output columns and a block of output rows and
+// streams the rows of u and lam like the 2-D stencil kernels: every lane
+// copies its own 16 bytes of each row into a ring in shared memory (cp.async)
+// groups ahead of use. At step p, row p-1 gets its q and w, row p-2 its
+// result; row p's differences with row p-1 stay in registers. In-row
+// neighbours come by shuffles.
+//
+// Bound for double: the FP64 pipe, 25 operations a cell. The two passes this
+// replaced (q and sum of differences to memory, then a gather) took about 60.
+// With the forward step's shared squares: forward and gradient of f64
+// 1024x1100, T=64, 18.7 -> 11.2 ms (GB300).
+template <class ST, typename T> struct GradPipe {
+  static constexpr int V = 16 / (int)sizeof(T);
+  static constexpr int COLS = 32 * V;
+  static constexpr int ML = (2 + V - 1) / V * V;             // window columns left of the outputs
+  static constexpr int WOUT = (COLS - ML - 2) / V * V;       // output columns per strip
+  static constexpr int NPH = 3, PG = 2;                      // rows per group, groups in flight
+  static constexpr unsigned ROWB = 1024;                     // ring row: u, then lam
+  static constexpr unsigned GROUP = NPH * ROWB, RING = (PG + 1) * GROUP;
+};
+constexpr int kGradWarps = 4;
 
-// gradient2d adjoint step (transposed linearised Jacobian) and dL/dnum partials
 template <class ST, typename T>
-__global__ void __launch_bounds__(kAdjThreads) grad_adj_kernel(const __grid_constant__ AdjGeom g, const T *u,
-                                                               const T *qp, const T *sdp, const T *lam_next,
-                                                               T *lam_prev, T *hg, double *part, T num,
-                                                               int want_coef) {
-  const long long cidx = (long long)blockIdx.x * kAdjThreads + threadIdx.x;
-  const int R = g.rad;
+__global__ void __launch_bounds__(kGradWarps * 32)
+    grad2d_kernel(const __grid_constant__ AdjGeom g, const T *u, const T *lam, T *lam_out, T *hg, double *part, T num,
+                  T eps, int want_coef, int nstrips, int nblocks, int sl) {
+  using GP = GradPipe<ST, T>;
+  using A = Arith<T>;
+  constexpr int V = GP::V, R = 1, NPH = GP::NPH, PG = GP::PG;
+  static_assert(ST::kKind != KIND_GRADIENT || ST::kRad == 1, "radius 1");
+  __shared__ __align__(128) unsigned char smem[kGradWarps * GP::RING];
+  __shared__ double red[kGradWarps];
+  wait_for_previous();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long gw = (long long)blockIdx.x * kGradWarps + wid;
   double pnum = 0.0;
-  if (cidx < g.cells) {
-    const int i = (int)(cidx / g.d1), j = (int)(cidx - (long long)(cidx / g.d1) * g.d1);
-    auto inter = [&](int a, int b) GBS_INL { return a >= R && a < g.d0 - R && b >= R && b < g.d1 - R; };
-    const long long o = cell_off(g, i, j, 0);
-    const bool yin = inter(i, j);
-    T acc = T(0);
-    if (yin) {
-      const T q = qp[o], ly = lam_next[o];
-      acc = ly * (T(1) - num * q * q * q * sdp[o]);
-      pnum = (double)(ly * q);
+  if (gw < (long long)nstrips * nblocks) {
+    const int strip = (int)(gw % nstrips), blk = (int)(gw / nstrips);
+    const int cs = R + strip * GP::WOUT, ce = min(cs + GP::WOUT, g.d1 - R);
+    const int own_lo = strip == 0 ? 0 : cs, own_hi = strip == nstrips - 1 ? g.d1 : ce;
+    const int el = cs + g.shift - GP::ML + lane * V;
+    const int col0 = el - g.shift;
+    const bool in_row = el >= 0 && el + V <= g.pitch;
+    bool on[V], inner[V], sum_col[V];
+    bool whole = true;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const int c = col0 + e;
+      on[e] = c >= 0 && c < g.d1;
+      inner[e] = c >= R && c < g.d1 - R;
+      sum_col[e] = c >= cs && c < ce;
+      whole = whole && sum_col[e];
     }
-    const T uy = u[o];
-    static_for<ST::kTerms>([&](auto TI) {
-      constexpr int t = decltype(TI)::value;
-      const int a = i - ST::kOff[t][0], b = j - ST::kOff[t][1];  // x with x + n = y
-      if (a >= 0 && a < g.d0 && b >= 0 && b < g.d1 && inter(a, b)) {
-        const long long ox = cell_off(g, a, b, 0);
-        const T qx = qp[ox];
-        acc = fma(lam_next[ox] * num * qx * qx * qx, u[ox] - uy, acc);
+    const int i0 = R + blk * sl, i1 = min(i0 + sl, g.d0 - R);
+    const int o0 = blk == 0 ? 0 : i0, o1 = blk == nblocks - 1 ? g.d0 : i1;  // result rows
+    const int pstart = max(0, o0 - 2), pend = min(g.d0, o1 + 2);
+    const int ng = (o1 + 2 - pstart + NPH - 1) / NPH;
+
+    unsigned char *my = smem + (size_t)wid * GP::RING + lane * 16;
+    const uint32_t my_s = smem_u32(my);
+    long long ld = (long long)pstart * g.pitch + el;
+    int ld_left = pend - pstart;
+    unsigned wr = 0, rd = 0;
+    auto request_group = [&]() GBS_INL {
+#pragma unroll
+      for (int ph = 0; ph < NPH; ++ph) {
+        if (in_row && ph < ld_left) {
+          cp_async16(my_s + wr + ph * GP::ROWB, u + ld);
+          cp_async16(my_s + wr + ph * GP::ROWB + 512, lam + ld);
+        }
+        ld += g.pitch;
       }
-    });
-    if (yin) {
-      lam_prev[o] = acc;
-    } else {
-      hg[o] += acc;
-      lam_prev[o] = T(0);
+      cp_async_commit();
+      ld_left -= NPH;
+      wr = wr + GP::GROUP == GP::RING ? 0u : wr + GP::GROUP;
+    };
+#pragma unroll 1
+    for (int k = 0; k < PG; ++k) request_group();
+
+    // rows p-1 (u1, l1), its differences with row p-2 (dv, their squares sv),
+    // row p-2's w and its result but for the edge to row p-1
+    T u1[V], l1[V], dv[V], sv[V], w2[V], acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) u1[e] = l1[e] = dv[e] = sv[e] = w2[e] = acc[e] = T(0);
+    int p = pstart;
+#pragma unroll 1
+    for (int k = 0; k < ng; ++k) {
+      request_group();
+      cp_async_wait<PG>();
+      static_for<NPH>([&](auto PHI) GBS_INL {
+        constexpr int ph = decltype(PHI)::value;
+        const int pp = p + ph;
+        T x[V], lx[V];
+        ld_vec<T, V>(x, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB));
+        ld_vec<T, V>(lx, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB + 512));
+        const bool row_on = pp < g.d0;
+        // off the grid u is 0, so that 0 * (u(x) - u(y)) is 0 there
+#pragma unroll
+        for (int e = 0; e < V; ++e) x[e] = row_on && on[e] ? x[e] : T(0);
+        const bool row_in = pp - 1 >= R && pp - 1 < g.d0 - R;  // row p-1 is interior
+        // horizontal edges of row p-1 (e: between columns e and e+1)
+        T dh[V], sh[V];
+        const T after = row_elem<V, V>(u1);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          dh[e] = A::sub(e + 1 < V ? u1[e + 1 < V ? e + 1 : e] : after, u1[e]);
+          sh[e] = A::mul(dh[e], dh[e]);
+        }
+        const T sleft = shfl_up(sh[V - 1], 1);
+        T dn[V], sn[V], w1[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          dn[e] = A::sub(x[e], u1[e]);
+          sn[e] = A::mul(dn[e], dn[e]);
+          const T s = A::add(A::add(A::add(A::add(eps, sv[e]), sn[e]), sh[e]), e > 0 ? sh[e > 0 ? e - 1 : 0] : sleft);
+          const T q = rsqrt_near(s);
+          const bool in = row_in && inner[e];
+          const T lv = in ? l1[e] : T(0);
+          w1[e] = in ? A::mul(A::mul(A::mul(num, lv), q), A::mul(q, q)) : T(0);
+          l1[e] = lv;
+          if (want_coef && in && sum_col[e] && pp - 1 >= i0 && pp - 1 < i1) pnum += (double)A::mul(lv, q);
+        }
+        // fluxes: horizontal edges of row p-1, vertical edges between rows p-2 and p-1
+        const T wafter = row_elem<V, V>(w1);
+        T fh[V], out[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) fh[e] = A::mul(A::add(w1[e], e + 1 < V ? w1[e + 1 < V ? e + 1 : e] : wafter), dh[e]);
+        const T fleft = shfl_up(fh[V - 1], 1);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const T fv = A::mul(A::add(w2[e], w1[e]), dv[e]);
+          out[e] = A::add(acc[e], fv);
+          acc[e] = A::add(l1[e], A::sub(A::sub(fh[e], e > 0 ? fh[e > 0 ? e - 1 : 0] : fleft), fv));
+          w2[e] = w1[e];
+          dv[e] = dn[e];
+          sv[e] = sn[e];
+          u1[e] = x[e];
+          l1[e] = lx[e];
+        }
+        const int q = pp - 2;  // the row whose result is complete
+        if (q >= o0 && q < o1) {
+          const long long o = (long long)q * g.pitch + el;
+          const bool in_rows = q >= R && q < g.d0 - R;
+          if (whole && in_rows) {
+            st_vec_global<T, V>(lam_out + o, out);
+          } else {
+#pragma unroll
+            for (int e = 0; e < V; ++e) {
+              const int c = col0 + e;
+              if (c < own_lo || c >= own_hi) continue;
+              if (in_rows && inner[e]) lam_out[o + e] = out[e];
+              else hg[o + e] += out[e];
+            }
+          }
+        }
+      });
+      p += NPH;
+      rd = rd + GP::GROUP == GP::RING ? 0u : rd + GP::GROUP;
     }
+    cp_async_wait<0>();
   }
   if (want_coef) {
-    __shared__ double red[kAdjThreads / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double v = pnum;
 #pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_down_sync(0xffffffffu, v, s);
-    if (lane == 0) red[w] = v;
+    for (int o = 16; o > 0; o >>= 1) pnum += __shfl_down_sync(0xffffffffu, pnum, o);
+    if (lane == 0) red[wid] = pnum;
     __syncthreads();
     if (threadIdx.x == 0) {
-      double s = 0.0;
+      double sum = 0.0;
 #pragma unroll
-      for (int ww = 0; ww < kAdjThreads / 32; ++ww) s += red[ww];
-      part[blockIdx.x] += s;
+      for (int k = 0; k < kGradWarps; ++k) sum += red[k];
+      part[blockIdx.x] += sum;
     }
   }
+}
+
+// The halo cells of `planes` planes, `stride` elements apart, from src (the
+// fixed boundary of recomputed states: launches never write it).
+template <typename T>
+__global__ void __launch_bounds__(kAdjThreads) copy_halo_kernel(const __grid_constant__ AdjGeom g, const T *src, T *dst,
+                                                                long long stride) {
+  const HaloPlan hp = halo_plan(g);
+  int i, j, c;
+  if (!halo_cell(g, hp, (long long)blockIdx.x * kAdjThreads + threadIdx.x, i, j, c)) return;
+  const long long o = g.dim == 2 ? cell_off(g, i, c, 0) : cell_off(g, i, j, c);
+  dst[(long long)blockIdx.y * stride + o] = src[o];
 }
 
 // zero the halo of a plane (lam_T's halo carries no gradient)
@@ -600,7 +701,7 @@ struct Workspace {
   int slots;            // stash planes: 2C (two chunk buffers) or fewer (revolve)
   bool revolve;         // chunks reversed by the binomial schedule
   size_t plane_bytes;
-  size_t off_cp, off_stash, off_lam, off_hg, off_q, off_sd, off_part, total;
+  size_t off_cp, off_stash, off_lam, off_hg, off_part, total;
 };
 
 // The stash holds two chunk buffers of C planes when slots >= 2C; with fewer
@@ -615,17 +716,13 @@ Workspace workspace_of(const gbs_desc *d, const Layout &L, int C, int slots) {
   w.revolve = slots < 2 * C;
   w.slots = w.revolve ? slots : 2 * C;
   w.plane_bytes = (size_t)L.plane * L.esize;
-  const long long cells = (long long)L.dims[0] * L.dims[1] * L.dims[2];
-  const bool grad = s->kind == 1;
-  w.nblocks = grad ? (int)((cells + kAdjThreads - 1) / kAdjThreads) : kCoefBlocks;
-  w.nt = grad ? 1 : std::min(s->nterms, kMaxCoefGrad);
+  w.nblocks = kCoefBlocks;
+  w.nt = s->kind == 1 ? 1 : std::min(s->nterms, kMaxCoefGrad);
   w.off_cp = 0;
   w.off_stash = w.off_cp + (size_t)w.ncp * w.plane_bytes;
   w.off_lam = w.off_stash + (size_t)(w.revolve ? w.slots + 2 : 2 * C) * w.plane_bytes;
   w.off_hg = w.off_lam + 2 * w.plane_bytes;
-  w.off_q = w.off_hg + w.plane_bytes;
-  w.off_sd = w.off_q + (grad ? w.plane_bytes : 0);
-  w.off_part = w.off_sd + (grad ? w.plane_bytes : 0);
+  w.off_part = w.off_hg + w.plane_bytes;
   w.total = w.off_part + (size_t)w.nblocks * w.nt * sizeof(double) + 256;
   return w;
 }
@@ -682,19 +779,19 @@ struct AdjKernels {
                          const std::vector<double> &, double, bool, cudaStream_t);
   cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t);
   cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t);
-  cudaError_t (*grad)(const AdjGeom &, const void *, void *, void *, const void *, void *, void *, double *, double,
-                      double, bool, cudaStream_t);
+  cudaError_t (*grad)(const AdjGeom &, const void *, const void *, void *, void *, double *, double, double, bool,
+                      cudaStream_t, bool);
 };
 
 // CTAs of a grid-stride kernel: one wave of resident CTAs (at most
 // kCoefBlocks, the rows of the partial-sum table), so that no partial second
 // wave repeats the per-CTA latency
 template <class K>
-int one_wave(K kernel) {
+int one_wave(K kernel, int threads) {
   int nb = 0, dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kAdjThreads, 0) != cudaSuccess || nb <= 0) {
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0) != cudaSuccess || nb <= 0) {
     (void)cudaGetLastError();
     return kCoefBlocks;
   }
@@ -706,18 +803,18 @@ int one_wave(K kernel) {
 // without products, stencils with as many terms) differ in registers and so
 // in resident CTAs, and a process may drive GPUs with different SM counts
 template <class K>
-int wave_cached(K kernel) {
+int wave_cached(K kernel, int threads = kAdjThreads) {
   static std::mutex mu;
   static std::map<std::pair<int, const void *>, int> cache;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     (void)cudaGetLastError();
-    return one_wave(kernel);
+    return one_wave(kernel, threads);
   }
   std::lock_guard<std::mutex> lk(mu);
   const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kernel));
   auto it = cache.find(key);
-  if (it == cache.end()) it = cache.emplace(key, one_wave(kernel)).first;
+  if (it == cache.end()) it = cache.emplace(key, one_wave(kernel, threads)).first;
   return it->second;
 }
 
@@ -726,6 +823,20 @@ unsigned halo_grid(const AdjGeom &g) {
   const HaloPlan h = halo_plan(g);
   const long long threads = h.na + h.rows_b * h.nseg * 32;
   return (unsigned)std::max<long long>(1, (threads + kAdjThreads - 1) / kAdjThreads);
+}
+
+// the halo of `planes` consecutive planes at dst from the plane src
+cudaError_t copy_halo(int dtype, const AdjGeom &g, const void *src, void *dst, int planes, cudaStream_t s) {
+  for (int k = 0; k < planes; k += 32768) {  // grid.y is at most 65535
+    const dim3 grid(halo_grid(g), (unsigned)std::min(planes - k, 32768));
+    if (dtype == GBS_F64)
+      copy_halo_kernel<double><<<grid, kAdjThreads, 0, s>>>(g, (const double *)src, (double *)dst + (size_t)k * g.plane,
+                                                            g.plane);
+    else
+      copy_halo_kernel<float><<<grid, kAdjThreads, 0, s>>>(g, (const float *)src, (float *)dst + (size_t)k * g.plane,
+                                                           g.plane);
+  }
+  return cudaGetLastError();
 }
 
 template <class ST, typename T>
@@ -792,20 +903,24 @@ cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *p
   }
 }
 
+// pdl: the stream's previous operation is another step (see Launch2D::pdl)
 template <class ST, typename T>
-cudaError_t run_grad(const AdjGeom &g, const void *u, void *q, void *sd, const void *lam_next, void *lam_prev,
-                     void *hg, double *part, double num, double eps, bool want_coef, cudaStream_t s) {
+cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam_out, void *hg, double *part,
+                     double num, double eps, bool want_coef, cudaStream_t s, bool pdl) {
   if constexpr (ST::kKind != KIND_GRADIENT) {
     return cudaErrorInvalidValue;
   } else {
-    const unsigned blocks = (unsigned)((g.cells + kAdjThreads - 1) / kAdjThreads);
-    grad_pre_kernel<ST, T><<<blocks, kAdjThreads, 0, s>>>(g, static_cast<const T *>(u), static_cast<T *>(q),
-                                                          static_cast<T *>(sd), (T)eps);
-    grad_adj_kernel<ST, T><<<blocks, kAdjThreads, 0, s>>>(
-        g, static_cast<const T *>(u), static_cast<const T *>(q), static_cast<const T *>(sd),
-        static_cast<const T *>(lam_next), static_cast<T *>(lam_prev), static_cast<T *>(hg), part, (T)num,
-        want_coef ? 1 : 0);
-    return cudaGetLastError();
+    using GP = GradPipe<ST, T>;
+    const int ni = g.d0 - 2, nstrips = (g.d1 - 2 + GP::WOUT - 1) / GP::WOUT;
+    const int wave = wave_cached(grad2d_kernel<ST, T>, kGradWarps * 32);
+    int sl = stream_rows_2d(nstrips, ni, 2, sizeof(T) == 8, (long long)wave * kGradWarps);
+    // one partial-sum row per CTA
+    while (((long long)nstrips * ((ni + sl - 1) / sl) + kGradWarps - 1) / kGradWarps > kCoefBlocks) ++sl;
+    const int nblocks = (ni + sl - 1) / sl;
+    const unsigned grid = (unsigned)(((long long)nstrips * nblocks + kGradWarps - 1) / kGradWarps);
+    return launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, pdl, g, static_cast<const T *>(u),
+                         static_cast<const T *>(lam), static_cast<T *>(lam_out), static_cast<T *>(hg), part, (T)num,
+                         (T)eps, want_coef ? 1 : 0, nstrips, nblocks, sl);
   }
 }
 
@@ -1091,8 +1206,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
   // one adjoint step lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_t) on state u_t
   auto step = [&](const char *u) -> gbs_status {
     if (gradient) {
-      CK(K.grad(g, u, ws + w.off_q, ws + w.off_sd, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps,
-                dev_coef_grad != nullptr, s),
+      CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s, false),
          "adjoint: gradient2d step");
     } else if (g.dim == 2 && sd->nterms <= kMaxCoefGrad) {
       CK(K.fused2d(g, lam[cur], u, lam[cur ^ 1], hg, part, coef, div, dev_coef_grad != nullptr, s),
@@ -1115,10 +1229,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     // Each chunk reversed by the binomial schedule over `slots` snapshot
     // planes and two work planes, all on `s`. The halo of every stash plane
     // is the fixed boundary (copied once; launches never write it).
-    for (int k = 0; k < w.slots + 2; ++k)
-      CK(cudaMemcpyAsync(stash + (size_t)k * w.plane_bytes, ws + w.off_cp, w.plane_bytes, cudaMemcpyDeviceToDevice,
-                         s),
-         "adjoint: stash");
+    CK(copy_halo(d->dtype, g, ws + w.off_cp, stash, w.slots + 2, s), "adjoint: stash");
     char *work0 = stash + (size_t)w.slots * w.plane_bytes;  // ping-pong partner of an advance
     char *work1 = work0 + w.plane_bytes;                     // target of a recompute without slots
     gbs_plan_info pi{};
@@ -1198,13 +1309,9 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       return cuda_fail(e, "adjoint: streams");
     }
     // the halo of every stash slot of both buffers: the fixed boundary (never rewritten)
-    for (int k = 0; k < 2 * w.C; ++k) {
-      e = cudaMemcpyAsync(stash + (size_t)k * w.plane_bytes, ws + w.off_cp, w.plane_bytes, cudaMemcpyDeviceToDevice,
-                          s);
-      if (e != cudaSuccess) {
-        release();
-        return cuda_fail(e, "adjoint: stash");
-      }
+    if ((e = copy_halo(d->dtype, g, ws + w.off_cp, stash, 2 * w.C, s)) != cudaSuccess) {
+      release();
+      return cuda_fail(e, "adjoint: stash");
     }
     cudaEventRecord(setup, s);
     cudaStreamWaitEvent(s2, setup, 0);

@@ -248,7 +248,7 @@ long long resident_warps_2d(int sid, int dtype, int fma, int b) {
 // instruction hide the rest). So short blocks for grids that leave the chip idle (a 128x96 grid
 // in blocks of 16 rows spent its time streaming them one by one on two SMs),
 // and for larger ones as many CTAs on every SM as on the busiest.
-static int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps) {
+int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps) {
   const int sms = sm_count();
   const int res = (int)std::max<long long>(1, (resident_warps > 0 ? resident_warps : 16LL * sms) /
                                                   (kWarpsPerCta2D * (long long)sms));

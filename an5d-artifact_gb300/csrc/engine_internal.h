@@ -52,6 +52,9 @@ gbs_status check_desc(const gbs_desc *d);
 Layout make_layout(const gbs_desc *d);
 std::vector<int> split_steps(int T, int bt);
 // resident_warps: warps the GPU holds at once for this kernel (0 = unknown)
+// rows per stream block of a 2-D launch of nstrips strips over ni rows whose
+// blocks overlap by br rows at each end
+int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps);
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident_warps);
 long long resident_warps_2d(int sid, int dtype, int fma, int b);
 // output columns per strip of the 2-D kernels (Pipe2D::WOUT): the window loses

@@ -234,31 +234,51 @@ __device__ __forceinline__ T term_next(T acc, T c, T a) {
   else return A::add(acc, A::mul(c, a));
 }
 
-// gradient2d.c:17-21: u + num / sqrt(eps + sum_n (u - u_n)^2), evaluated as
-// C evaluates it: the differences and squares summed in T, each rounded, then
-// (since `1.0f / sqrt(x)` calls the double sqrt) the root, the quotient and
-// the final sum in double, rounded once to T (exact mode). Both modes form
-// the sum of squares this way: the update amplifies rounding where
-// neighbours agree, so even fusing the squares drifts past the 1e-5 parity
-// bound within ten steps. FMA mode (FAST) replaces the double root and
-// quotient, which run on the FP64 pipe at 1/64 of the FP32 rate.
-template <typename T, int NN, bool FAST = false>
-__device__ __forceinline__ T gradient_update(T u, const T (&nb)[NN], T eps, T num) {
-  using A = Arith<T>;
-  T s = eps;
-#pragma unroll
-  for (int n = 0; n < NN; ++n) {
-    const T d = A::sub(u, nb[n]);
-    s = A::add(s, A::mul(d, d));
-  }
+// 1/sqrt(s) for double on few FP64 operations: the hardware's approximation
+// (rsqrt.approx.ftz.f64, from the upper word of s) and one third-order step of
+// Householder's iteration, y (1 + e/2 + 3 e^2/8) with e = 1 - s y^2, which
+// cubes its relative error. For s in [2^-100, 2^100]; 5 FP64 operations
+// (two Newton steps from a float estimate: 8, two conversions and two
+// comparisons, all on the FP64 pipe).
+__device__ __forceinline__ double rsqrt_core(double s) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double e = __fma_rn(-__dmul_rn(s, y), y, 1.0);
+  return __fma_rn(__dmul_rn(y, e), __fma_rn(0.375, e, 0.5), y);
+}
+// s in [2^-100, 2^100): one integer comparison of its upper word
+__device__ __forceinline__ bool rsqrt_range(double s) {
+  return (unsigned)(__double2hiint(s) - ((1023 - 100) << 20)) < (200u << 20);
+}
+__device__ __noinline__ inline double rsqrt_rare(double s) { return 1.0 / sqrt(s); }
+// 1/sqrt(s) to about one rounding
+__device__ __forceinline__ double rsqrt_near(double s) { return rsqrt_range(s) ? rsqrt_core(s) : rsqrt_rare(s); }
+__device__ __forceinline__ float rsqrt_near(float s) {
+  const float y = rsqrtf(s);
+  const float p = __fmul_rn(s, y);
+  float e = __fmaf_rn(-p, y, 1.0f);
+  e = __fmaf_rn(-__fmaf_rn(s, y, -p), y, e);  // 1 - s y^2, the product s y exact
+  return s > 0.0f && s < 3e38f ? __fmaf_rn(__fmul_rn(0.5f, y), e, y) : y;
+}
+
+// gradient2d.c:17-21: u + num / sqrt(s), s = eps + sum_n (u - u_n)^2 (formed by
+// the caller, every difference, square and sum rounded separately in both
+// modes: the update amplifies rounding where neighbours agree, so even fusing
+// the squares drifts past the 1e-5 parity bound within ten steps), evaluated
+// as C evaluates it in exact mode: since `1.0f / sqrt(x)` calls the double
+// sqrt, the root, the quotient and the final sum in double, rounded once to T.
+// FMA mode (FAST) replaces the double root and quotient, which run on the
+// FP64 pipe at 1/64 of the FP32 rate.
+template <typename T, bool FAST>
+__device__ __forceinline__ T gradient_finish(T u, T s, T num) {
   if constexpr (FAST && std::is_same<T, float>::value) {
     // FMA mode, float, all on the FP32 pipe. q = num / sqrt(s) as an
-    // unevaluated pair qh + ql: y0 = RN(1/sqrt(s)), then one Newton
+    // unevaluated pair qh + ql: y0 = an estimate of 1/sqrt(s), then one Newton
     // correction 1/sqrt(s) ~ y0 (1 + e/2) whose residual e = 1 - s y0^2 is
     // formed exactly with FMA (s y0 = p + pe). u + qh + ql is then rounded
     // once through Knuth's TwoSum, like exact mode's single rounding of the
     // double sum (they differ only within ~2^-20 ulp of a rounding midpoint).
-    const float y0 = __frsqrt_rn(s);
+    const float y0 = rsqrtf(s);
     const float p = __fmul_rn(s, y0);
     const float pe = __fmaf_rn(s, y0, -p);
     float e = __fmaf_rn(-p, y0, 1.0f);
@@ -271,20 +291,7 @@ __device__ __forceinline__ T gradient_update(T u, const T (&nb)[NN], T eps, T nu
     const float err = __fadd_rn(__fsub_rn(u, __fsub_rn(t, bv)), __fsub_rn(qh, bv));
     return __fadd_rn(t, __fadd_rn(err, ql));
   } else if constexpr (FAST) {
-    // FMA mode, double: Newton-Raphson iteration for 1/sqrt(s),
-    // y <- y + y (1 - s y^2) / 2, from a single-precision estimate (relative
-    // error about 2^-22); each step squares the error, so two steps reach
-    // double precision with five FP64 operations instead of a division and
-    // a square root. Outside the guarded range: division and square root.
-    if (s >= 1e-30 && s <= 1e30) {
-      double y = (double)rsqrtf((float)s);
-      double h = fma(-s * y, y, 1.0);
-      y = fma(0.5 * y, h, y);
-      h = fma(-s * y, y, 1.0);
-      y = fma(0.5 * y, h, y);
-      return u + num * y;
-    }
-    return u + num / sqrt(s);
+    return __fma_rn(num, rsqrt_near(s), u);
   } else {
     const double q = __ddiv_rn((double)num, __dsqrt_rn((double)s));
     const double r = __dadd_rn((double)u, q);

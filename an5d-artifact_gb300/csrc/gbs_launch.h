@@ -38,11 +38,11 @@ struct Launch3D {
   bool pdl;           // as in Launch2D
 };
 
-// kern<<<grid, block, smem, stream>>>(p), with the programmatic-dependent-launch
-// attribute when pdl is set
-template <class P>
-cudaError_t launch_kernel(void (*kern)(P), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, bool pdl,
-                          const P &p) {
+// kern<<<grid, block, smem, stream>>>(args...), with the
+// programmatic-dependent-launch attribute when pdl is set
+template <class... P, class... Args>
+cudaError_t launch_kernel(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+                          bool pdl, Args &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
@@ -53,7 +53,7 @@ cudaError_t launch_kernel(void (*kern)(P), unsigned grid, unsigned block, size_t
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, p);
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 using Launch2DFn = cudaError_t (*)(const Launch2D &, cudaStream_t);

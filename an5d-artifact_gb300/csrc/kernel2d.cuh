@@ -192,12 +192,13 @@ enum Care2D : int {
 };
 
 // One fused time level: the level-(l) row x arrives, the level-(l+1) row q
-// leaves in x.
+// leaves in x. up (gradient2d): the squared differences between rows q-1 and q,
+// which the step of row q-1 formed.
 // The sums of the few overlap rows that no output needs are computed all the
 // same: a test per row and level costs more than it saves, on the FP64 pipe
 // too (star2d1r f64 16384^2 2755 us a step with it, 2444 without).
 template <class ST, class PP, typename T, bool FMA, int CARE, int PH>
-__device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&x)[PP::V], int q,
+__device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&up)[PP::V], T (&x)[PP::V], int q,
                                         const bool (&fixed)[PP::V], const CarryRing<PP> &carry,
                                         const Params2D<T, ST::kTerms> &p) {
   constexpr int R = ST::kRad;
@@ -211,19 +212,31 @@ __device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&x)[PP::
     for (int e = 0; e < V; ++e) win[slot2d<PP>(PH, 2 * R)][e] = x[e];
     constexpr int cslot = slot2d<PP>(PH, R);
     if constexpr (ST::kKind == KIND_GRADIENT) {
-      T ext[V + 2 * R];
-      extend_row<ST, V, 0>(ext, win[cslot]);
-      static_for<V>([&](auto EI) GBS_INL {
-        constexpr int e = decltype(EI)::value;
-        T nb[ST::kTerms];
-        static_for<ST::kTerms>([&](auto TI) GBS_INL {
-          constexpr int t = decltype(TI)::value;
-          constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-          if constexpr (di == 0) nb[t] = ext[R + e + dj];
-          else nb[t] = win[slot2d<PP>(PH, R + di)][e];
-        });
-        y[e] = gradient_update<T, ST::kTerms, FMA>(win[cslot][e], nb, p.eps, p.coef[0]);
-      });
+      // the squared differences in source order (up, down, right, left). Each
+      // is one of two cells' (u - u_n and u_n - u are exact negatives, so the
+      // squares are equal): the upper one was the row above's lower one, the
+      // left one is the left neighbour's right one. 14 FP64 operations a
+      // cell instead of 25.
+      static_assert(ST::kTerms == 4 && R == 1 && ST::kOff[0][0] == -1 && ST::kOff[1][0] == 1 &&
+                        ST::kOff[2][1] == 1 && ST::kOff[3][1] == -1, "neighbours: up, down, right, left");
+      const T(&c)[V] = win[cslot];
+      const T(&below)[V] = win[slot2d<PP>(PH, 2)];
+      const T after = row_elem<V, V>(c);
+      T sr[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const T d = A::sub(c[e], e + 1 < V ? c[e + 1 < V ? e + 1 : e] : after);
+        sr[e] = A::mul(d, d);
+      }
+      const T sl = shfl_up(sr[V - 1], 1);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const T d = A::sub(c[e], below[e]);
+        const T sd = A::mul(d, d);
+        const T s = A::add(A::add(A::add(A::add(p.eps, up[e]), sd), sr[e]), e > 0 ? sr[e > 0 ? e - 1 : 0] : sl);
+        up[e] = sd;
+        y[e] = gradient_finish<T, FMA>(c[e], s, p.coef[0]);
+      }
     } else {
       // the direct form serves stencils whose off-centre rows are read at
       // the centre column only (stars, star2d4r): one extended row
@@ -360,6 +373,12 @@ __device__ __forceinline__ void warp_item2d(const Params2D<T, ST::kTerms> &p, in
 #pragma unroll
       for (int e = 0; e < V; ++e) win[l][w][e] = T(0);
 
+  T up[B][V];  // see level2d
+#pragma unroll
+  for (int l = 0; l < B; ++l)
+#pragma unroll
+    for (int e = 0; e < V; ++e) up[l][e] = T(0);
+
   unsigned rd = 0;                               // byte offset of the group being computed
   T *st = p.dst + (long long)(pstart - B * R) * p.pitch + el;  // row the last level stores in the first step
   T *ss = STASH ? p.stash + (long long)pstart * p.pitch + el : nullptr;
@@ -378,7 +397,7 @@ __device__ __forceinline__ void warp_item2d(const Params2D<T, ST::kTerms> &p, in
       ld_ring<PP>(x, my + rd + (unsigned)ph * PP::ROWB);
       static_for<B>([&](auto LI) GBS_INL {
         constexpr int l = decltype(LI)::value;
-        level2d<ST, PP, T, FMA, care, ph>(win[l], x, pp - (l + 1) * R, fixed, carry, p);
+        level2d<ST, PP, T, FMA, care, ph>(win[l], up[l], x, pp - (l + 1) * R, fixed, carry, p);
         if constexpr (STASH && l + 1 < B) {
           const unsigned ql = (unsigned)(pp - (l + 1) * R - i0);
           if (ql < nout) {
