@@ -43,23 +43,13 @@
 #include <cstring>
 #include <vector>
 
-#include "engine_internal.h"
+#include "adjoint_internal.h"
 #include "gbs_device.cuh"
 
 namespace gbs {
 namespace {
 
 constexpr int kAdjThreads = 256;
-constexpr int kMaxCoefGrad = 32;  // coefficient gradients for stencils of at most this many terms
-constexpr int kCoefBlocks = 1024;  // CTAs of the coefficient kernel (one partial row each)
-
-struct AdjGeom {
-  long long pitch, plane;  // elements
-  int d0, d1, d2, dim, shift, rad;
-  int rows, last;          // rows per plane (d0 or d0*d1), cells per row
-  long long cells;         // d0*d1*d2
-};
-
 __device__ __forceinline__ long long cell_off(const AdjGeom &g, int i, int j, int k) {
   return g.dim == 2 ? (long long)i * g.pitch + g.shift + j
                     : ((long long)i * g.d1 + j) * g.pitch + g.shift + k;
@@ -242,204 +232,6 @@ __global__ void __launch_bounds__(kAdjThreads) coef_kernel(const __grid_constant
 #pragma unroll
     for (int ww = 0; ww < kAdjThreads / 32; ++ww) s += red[ww][threadIdx.x];
     part[(size_t)blockIdx.x * NT + threadIdx.x] += s * (double)inv_div;
-  }
-}
-
-// The elements of one row that a segment's end lanes cannot take from a
-// neighbouring lane: left[x + R] for x in [-R, 0) (lanes within R/V of the
-// warp's start) and right[x - V] for x in [V, V + R) (lanes within R/V of
-// its end), relative to the lane's first column; loaded once, when the row
-// enters the lane's register window, instead of once per term and use.
-template <typename T, int V, int R> struct RowEdges {
-  T left[R], right[R];
-};
-template <typename T, int V, int R>
-__device__ __forceinline__ void load_edges(RowEdges<T, V, R> &ed, const T *p, long long rowbase, int lane) {
-  static_for<R>([&](auto XI) {
-    constexpr int x = -1 - decltype(XI)::value;  // -1 .. -R
-    constexpr int dl = (-x + V - 1) / V;
-    if (lane < dl) ed.left[x + R] = p[rowbase + x];
-  });
-  static_for<R>([&](auto XI) {
-    constexpr int x = V + decltype(XI)::value;   // V .. V+R-1
-    constexpr int dl = x / V;
-    if (lane >= 32 - dl) ed.right[x - V] = p[rowbase + x];
-  });
-}
-// Element x (relative to the lane's first column, x in [-R, V+R)) of the row
-// at window position P: from the lane's own vector, from a lane up to R/V
-// away, or, for the lanes whose source lane lies outside the warp, from the
-// row's cached edges
-template <int V, int R, int P, int X, typename T, int NWIN>
-__device__ __forceinline__ T row_value_cached(const T (&rows)[NWIN][V], const RowEdges<T, V, R> (&ed)[NWIN],
-                                              int lane) {
-  T v = row_elem<V, X>(rows[P]);
-  if constexpr (X < 0) {
-    constexpr int dl = (-X + V - 1) / V;
-    if (lane < dl) v = ed[P].left[X + R];
-  } else if constexpr (X >= V) {
-    constexpr int dl = X / V;
-    if (lane >= 32 - dl) v = ed[P].right[X - V];
-  }
-  return v;
-}
-
-// rows of lam (and u) the adjoint step loads per batch: one memory latency
-// per batch of output rows instead of one per row. The window holds 2R + K
-// rows of each array, so the batch shrinks with the radius and for double
-// (radius 1 float at K = 4 takes 116 registers with the coefficient
-// products; larger windows spill).
-template <typename T, int R>
-constexpr int adj_batch() {
-  if (sizeof(T) == 4) return R == 1 ? 4 : (R == 2 ? 2 : 1);
-  return R == 1 ? 2 : 1;
-}
-
-// 2-D linear adjoint step, fused: lam_out(y) = sum_k c_k/d lam(y - o_k) on
-// the interior (lam is zero on the halo; lam_out's halo is never written),
-// with WANT_COEF the products lam(y) u(y + o_k) / d summed per thread and
-// reduced per CTA into part[blockIdx.x][k], and hg(h) += the transposed sum
-// at every halo cell h. One launch per step instead of the transposed engine
-// step, the halo kernel and the product kernel: 2-D grids are small enough
-// that a step is bound by kernel latency. The first `interior_blocks` CTAs
-// take work units of one 32*V-column segment by `rows` interior rows: each
-// lane streams its aligned 16-byte vector of V columns down the rows,
-// keeping the rows of lam (and of u) that the next batch of output rows
-// needs in registers, so that every row is loaded once per unit and the
-// loads of a batch of rows are in flight together (a unit of a few rows per
-// warp is otherwise a chain of dependent memory latencies); in-row
-// neighbours come from the lanes up to R/V away (the warp's edge lanes load
-// theirs). The CTAs after them take the halo cells (one thread each).
-template <class ST, typename T, bool WANT_COEF>
-__global__ void __launch_bounds__(kAdjThreads) adj2d_kernel(const __grid_constant__ AdjGeom g,
-                                                            const T *__restrict__ lam, const T *__restrict__ u,
-                                                            T *__restrict__ lam_out, T *__restrict__ hg,
-                                                            double *__restrict__ part,
-                                                            const __grid_constant__ LinCoef<T, ST::kTerms> cf,
-                                                            T inv_div, int interior_blocks, int rows) {
-  constexpr int NT = ST::kTerms;
-  constexpr int NP = WANT_COEF ? NT : 1;
-  constexpr int V = 16 / sizeof(T);
-  constexpr int R = ST::kRad;
-  constexpr int SEG = 32 * V;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if ((int)blockIdx.x >= interior_blocks) {
-    const HaloPlan hp = halo_plan(g);
-    int i, j, c;
-    if (halo_cell(g, hp, (long long)(blockIdx.x - interior_blocks) * kAdjThreads + threadIdx.x, i, j, c))
-      halo_update<ST, T>(g, lam, hg, cf, i, j, c);
-    return;
-  }
-  T acc[NP];
-#pragma unroll
-  for (int t = 0; t < NP; ++t) acc[t] = T(0);
-  const int width = g.last - 2 * R;
-  const int nseg = (width + SEG - 1) / SEG;
-  const int ni = g.d0 - 2 * R;
-  const int nblk = (ni + rows - 1) / rows;
-  const long long units = (long long)nblk * nseg;
-  const long long nwarps = (long long)interior_blocks * (kAdjThreads / 32);
-  for (long long un = (long long)blockIdx.x * (kAdjThreads / 32) + w; un < units; un += nwarps) {
-    const int blk = (int)(un / nseg), seg = (int)(un - (long long)blk * nseg);
-    const int ia = R + blk * rows, ib = min(ia + rows, g.d0 - R);  // output rows [ia, ib)
-    const int c0 = R + seg * SEG + lane * V;        // the lane's first column; 16-byte aligned
-    const int nvalid = min(V, g.last - R - c0);     // columns of the group inside the interior
-    const long long col = (long long)g.shift + c0;
-    // windows of rows i-R .. i+R+K-1 (position p holds row i-R+p), refilled
-    // K rows at a time: the K new rows of lam (and u) are loaded together
-    constexpr int K = adj_batch<T, R>();
-    constexpr int NWIN = 2 * R + K;
-    T lw[NWIN][V], uw[WANT_COEF ? NWIN : 1][V];
-    RowEdges<T, V, R> le[NWIN], ue[WANT_COEF ? NWIN : 1];  // the segment-end elements of each row
-    static_for<2 * R>([&](auto PI) {
-      constexpr int pp = decltype(PI)::value;  // rows ia-R .. ia+R-1
-      const long long rb = (long long)(ia - R + pp) * g.pitch + col;
-      ld_vec<T, V>(lw[pp], lam + rb);
-      load_edges<T, V, R>(le[pp], lam, rb, lane);
-      if constexpr (WANT_COEF) {
-        ld_vec<T, V>(uw[pp], u + rb);
-        load_edges<T, V, R>(ue[pp], u, rb, lane);
-      }
-    });
-#pragma unroll 1
-    for (int i = ia; i < ib; i += K) {
-      // load rows i+R .. i+R+K-1 (those below ib+R; the rest are not read)
-      static_for<K>([&](auto KI) {
-        constexpr int kk = decltype(KI)::value;
-        if (i + kk < ib) {
-          const long long rb = (long long)(i + R + kk) * g.pitch + col;
-          ld_vec<T, V>(lw[2 * R + kk], lam + rb);
-          load_edges<T, V, R>(le[2 * R + kk], lam, rb, lane);
-          if constexpr (WANT_COEF) {
-            ld_vec<T, V>(uw[2 * R + kk], u + rb);
-            load_edges<T, V, R>(ue[2 * R + kk], u, rb, lane);
-          }
-        }
-      });
-      static_for<K>([&](auto KI) {
-        constexpr int kk = decltype(KI)::value;  // output row i+kk: window positions kk .. kk+2R
-        if (i + kk < ib) {
-          const long long base = (long long)(i + kk) * g.pitch + col;
-          T sv[V];
-#pragma unroll
-          for (int e = 0; e < V; ++e) sv[e] = T(0);
-          static_for<NT>([&](auto TI) {
-            constexpr int t = decltype(TI)::value;
-            constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-            static_for<V>([&](auto EI) {
-              constexpr int e = decltype(EI)::value;
-              sv[e] = fma(cf.c[t], row_value_cached<V, R, kk + R - di, e - dj>(lw, le, lane), sv[e]);
-            });
-          });
-          if constexpr (WANT_COEF) {
-            static_for<NT>([&](auto TI) {
-              constexpr int t = decltype(TI)::value;
-              constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1];
-              static_for<V>([&](auto EI) {
-                constexpr int e = decltype(EI)::value;
-                const T uv = row_value_cached<V, R, kk + R + di, e + dj>(uw, ue, lane);
-                if (e < nvalid) acc[t] = fma(lw[kk + R][e], uv, acc[t]);
-              });
-            });
-          }
-          if (nvalid == V) {
-            st_vec<T, V>(lam_out + base, sv);
-          } else {
-#pragma unroll
-            for (int e = 0; e < V; ++e)
-              if (e < nvalid) lam_out[base + e] = sv[e];
-          }
-        }
-      });
-      // slide by K: rows i+K-R .. i+K+R-1 to positions 0 .. 2R-1
-      static_for<2 * R>([&](auto PI) {
-        constexpr int pp = decltype(PI)::value;
-#pragma unroll
-        for (int e = 0; e < V; ++e) {
-          lw[pp][e] = lw[pp + K][e];
-          if constexpr (WANT_COEF) uw[pp][e] = uw[pp + K][e];
-        }
-        le[pp] = le[pp + K];
-        if constexpr (WANT_COEF) ue[pp] = ue[pp + K];
-      });
-    }
-  }
-  if constexpr (WANT_COEF) {
-    __shared__ double red[kAdjThreads / 32][NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      T v = acc[t];
-#pragma unroll
-      for (int sh = 16; sh > 0; sh >>= 1) v += __shfl_down_sync(0xffffffffu, v, sh);
-      if (lane == 0) red[w][t] = (double)v;
-    }
-    __syncthreads();
-    if (threadIdx.x < NT) {
-      double sum = 0.0;
-#pragma unroll
-      for (int ww = 0; ww < kAdjThreads / 32; ++ww) sum += red[ww][threadIdx.x];
-      part[(size_t)blockIdx.x * NT + threadIdx.x] += sum * (double)inv_div;
-    }
   }
 }
 
@@ -716,7 +508,7 @@ Workspace workspace_of(const gbs_desc *d, const Layout &L, int C, int slots) {
   w.revolve = slots < 2 * C;
   w.slots = w.revolve ? slots : 2 * C;
   w.plane_bytes = (size_t)L.plane * L.esize;
-  w.nblocks = kCoefBlocks;
+  w.nblocks = kAdjPartRows;
   w.nt = s->kind == 1 ? 1 : std::min(s->nterms, kMaxCoefGrad);
   w.off_cp = 0;
   w.off_stash = w.off_cp + (size_t)w.ncp * w.plane_bytes;
@@ -775,48 +567,11 @@ bool transposed_coefficients(const gbs_stencil_def_t *s, const std::vector<doubl
 
 // kernels of one stencil and dtype
 struct AdjKernels {
-  cudaError_t (*fused2d)(const AdjGeom &, const void *, const void *, void *, void *, double *,
-                         const std::vector<double> &, double, bool, cudaStream_t);
   cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t);
   cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t);
   cudaError_t (*grad)(const AdjGeom &, const void *, const void *, void *, void *, double *, double, double, bool,
                       cudaStream_t, bool);
 };
-
-// CTAs of a grid-stride kernel: one wave of resident CTAs (at most
-// kCoefBlocks, the rows of the partial-sum table), so that no partial second
-// wave repeats the per-CTA latency
-template <class K>
-int one_wave(K kernel, int threads) {
-  int nb = 0, dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, 0) != cudaSuccess || nb <= 0) {
-    (void)cudaGetLastError();
-    return kCoefBlocks;
-  }
-  return std::max(1, std::min(kCoefBlocks, nb * sms));
-}
-
-// one_wave(kernel) on the current device, computed once per (device
-// ordinal, kernel): kernels of the same signature (the variants with and
-// without products, stencils with as many terms) differ in registers and so
-// in resident CTAs, and a process may drive GPUs with different SM counts
-template <class K>
-int wave_cached(K kernel, int threads = kAdjThreads) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void *>, int> cache;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return one_wave(kernel, threads);
-  }
-  std::lock_guard<std::mutex> lk(mu);
-  const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kernel));
-  auto it = cache.find(key);
-  if (it == cache.end()) it = cache.emplace(key, one_wave(kernel, threads)).first;
-  return it->second;
-}
 
 // one thread per halo cell of the interior rows, one warp per segment of an all-halo row
 unsigned halo_grid(const AdjGeom &g) {
@@ -854,49 +609,12 @@ cudaError_t run_halo(const AdjGeom &g, const void *lam, void *hg, const std::vec
 }
 
 template <class ST, typename T>
-cudaError_t run_fused2d(const AdjGeom &g, const void *lam, const void *u, void *lam_out, void *hg, double *part,
-                        const std::vector<double> &coef, double div, bool want_coef, cudaStream_t s) {
-  if constexpr (ST::kKind == KIND_GRADIENT || ST::kDim != 2 || ST::kTerms > kMaxCoefGrad) {
-    return cudaErrorInvalidValue;
-  } else {
-    LinCoef<T, ST::kTerms> cf;
-    const double dv = ST::kHasDiv ? div : 1.0;
-    for (int t = 0; t < ST::kTerms; ++t) cf.c[t] = (T)(coef[t] / dv);
-    const T inv = (T)(1.0 / dv);
-    const HaloPlan hp = halo_plan(g);
-    const long long halo_threads = hp.na + hp.rows_b * hp.nseg * 32;
-    const unsigned halo_blocks = (unsigned)((halo_threads + kAdjThreads - 1) / kAdjThreads);
-    const int wave_c = wave_cached(adj2d_kernel<ST, T, true>);
-    const int wave_n = wave_cached(adj2d_kernel<ST, T, false>);
-    // rows per work unit: about one unit per resident warp, at least 4 rows
-    // so that the 2R rows each unit loads to fill its window stay a minor cost
-    constexpr int SEG = 32 * (16 / sizeof(T));
-    const long long nseg = (g.last - 2 * ST::kRad + SEG - 1) / SEG;
-    const int ni = g.d0 - 2 * ST::kRad;
-    auto rows_for = [&](int wave) {
-      const long long warps = (long long)wave * (kAdjThreads / 32);
-      const long long per = (ni * nseg + warps - 1) / std::max(1LL, warps);
-      return (int)std::max<long long>(4, std::min<long long>(ni, per));
-    };
-    if (want_coef)
-      adj2d_kernel<ST, T, true><<<wave_c + halo_blocks, kAdjThreads, 0, s>>>(
-          g, static_cast<const T *>(lam), static_cast<const T *>(u), static_cast<T *>(lam_out), static_cast<T *>(hg),
-          part, cf, inv, wave_c, rows_for(wave_c));
-    else
-      adj2d_kernel<ST, T, false><<<wave_n + halo_blocks, kAdjThreads, 0, s>>>(
-          g, static_cast<const T *>(lam), static_cast<const T *>(u), static_cast<T *>(lam_out), static_cast<T *>(hg),
-          part, cf, inv, wave_n, rows_for(wave_n));
-    return cudaGetLastError();
-  }
-}
-
-template <class ST, typename T>
 cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *part, double div, cudaStream_t s) {
   if constexpr (ST::kKind == KIND_GRADIENT || ST::kTerms > kMaxCoefGrad) {
     return cudaErrorInvalidValue;
   } else {
     const double dv = ST::kHasDiv ? div : 1.0;
-    const int wave = wave_cached(coef_kernel<ST, T>);
+    const int wave = std::min(kAdjPartRows, adj_wave(reinterpret_cast<const void *>(coef_kernel<ST, T>), kAdjThreads, 0));
     coef_kernel<ST, T><<<wave, kAdjThreads, 0, s>>>(g, static_cast<const T *>(lam), static_cast<const T *>(u), part,
                                                     (T)(1.0 / dv));
     return cudaGetLastError();
@@ -912,10 +630,10 @@ cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam
   } else {
     using GP = GradPipe<ST, T>;
     const int ni = g.d0 - 2, nstrips = (g.d1 - 2 + GP::WOUT - 1) / GP::WOUT;
-    const int wave = wave_cached(grad2d_kernel<ST, T>, kGradWarps * 32);
+    const int wave = adj_wave(reinterpret_cast<const void *>(grad2d_kernel<ST, T>), kGradWarps * 32, 0);
     int sl = stream_rows_2d(nstrips, ni, 2, sizeof(T) == 8, (long long)wave * kGradWarps);
     // one partial-sum row per CTA
-    while (((long long)nstrips * ((ni + sl - 1) / sl) + kGradWarps - 1) / kGradWarps > kCoefBlocks) ++sl;
+    while (((long long)nstrips * ((ni + sl - 1) / sl) + kGradWarps - 1) / kGradWarps > kAdjPartRows) ++sl;
     const int nblocks = (ni + sl - 1) / sl;
     const unsigned grid = (unsigned)(((long long)nstrips * nblocks + kGradWarps - 1) / kGradWarps);
     return launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, pdl, g, static_cast<const T *>(u),
@@ -926,17 +644,31 @@ cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam
 
 AdjKernels adj_kernels(int sid, int dtype) {
   switch (sid) {
-#define GBS_ADJ(id, S)                                                                            \
-  case id:                                                                                         \
-    return dtype == GBS_F64                                                                       \
-               ? AdjKernels{&run_fused2d<S, double>, &run_halo<S, double>, &run_coef<S, double>,      \
-                            &run_grad<S, double>}                                                       \
-               : AdjKernels{&run_fused2d<S, float>, &run_halo<S, float>, &run_coef<S, float>, &run_grad<S, float>};
+#define GBS_ADJ(id, S)                                                               \
+  case id:                                                                            \
+    return dtype == GBS_F64                                                          \
+               ? AdjKernels{&run_halo<S, double>, &run_coef<S, double>, &run_grad<S, double>} \
+               : AdjKernels{&run_halo<S, float>, &run_coef<S, float>, &run_grad<S, float>};
     GBS_FOR_EACH_STENCIL(GBS_ADJ)
 #undef GBS_ADJ
     default:
-      return AdjKernels{nullptr, nullptr, nullptr, nullptr};
+      return AdjKernels{nullptr, nullptr, nullptr};
   }
+}
+
+// launchers of the built stencil with sd's offsets, term by term
+AdjPicks2D adj2d_picks(const gbs_stencil_def_t *sd, int dtype) {
+#define GBS_ADJ2D(id)                                                                        \
+  {                                                                                          \
+    const gbs_stencil_def_t *o = stencil_def(id);                                            \
+    bool same = o->dim == sd->dim && o->kind == sd->kind && o->nterms == sd->nterms;         \
+    for (int t = 0; same && t < o->nterms; ++t)                                              \
+      same = o->terms[t].di == sd->terms[t].di && o->terms[t].dj == sd->terms[t].dj;         \
+    if (same) return dtype == GBS_F64 ? adj2d_picks_##id##_d() : adj2d_picks_##id##_f();     \
+  }
+  GBS_FOR_EACH_ADJ2D(GBS_ADJ2D)
+#undef GBS_ADJ2D
+  return AdjPicks2D{};
 }
 
 // ---------------------------------------------------------------------------
@@ -1051,6 +783,28 @@ gbs_status on_branches(int n, cudaStream_t stream, F run) {
 }
 
 }  // namespace
+
+// computed once per (device ordinal, kernel): a process may drive GPUs with
+// different SM counts
+int adj_wave(const void *kernel, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, int> cache;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    dev = 0;
+  }
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = cache.find({dev, kernel});
+  if (it != cache.end()) return it->second;
+  int nb = 0, sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess || nb <= 0) {
+    (void)cudaGetLastError();
+    return kAdjPartRows;
+  }
+  return cache.emplace(std::make_pair(dev, kernel), nb * sms).first->second;
+}
 }  // namespace gbs
 
 using namespace gbs;
@@ -1203,14 +957,39 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
   CK(cudaMemsetAsync(hg, 0, w.plane_bytes, s), "adjoint: memset");
   CK(cudaMemsetAsync(part, 0, (size_t)w.nblocks * w.nt * sizeof(double), s), "adjoint: memset");
   int cur = 0;
+  const bool blocked = !gradient && g.dim == 2 && sd->nterms <= kMaxCoefGrad;  // adjoint2d.cu
+  const AdjPicks2D P2 = blocked ? adj2d_picks(sd, d->dtype) : AdjPicks2D{};
+  if (blocked && !P2.step[0][1]) return fail(GBS_ERR_UNSUPPORTED, "no 2-D adjoint step built for %s", sd->name);
+  const int want = dev_coef_grad ? 1 : 0;
+  // steps of one launch when `left` remain
+  auto degree = [&](int left) {
+    for (int b = std::min(left, kAdjMaxB); b > 1; --b)
+      if (P2.step[want][b]) return b;
+    return 1;
+  };
+  // b adjoint steps lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_{t+1-b}), u = the state u_t (u_{t-1} one plane
+  // before it, ...); b > 1 for blocked stencils only. follows: the stream's previous operation is such a step
+  auto steps = [&](const char *u, int b, bool follows) -> gbs_status {
+    AdjStep2D a{};
+    a.g = &g;
+    a.lam = lam[cur];
+    a.u = u;
+    a.lam_out = lam[cur ^ 1];
+    a.hg = hg;
+    a.part = part;
+    a.coef = coef.data();
+    a.div = sd->divisor ? div : 1.0;
+    a.pdl = follows;
+    CK(P2.step[want][b](a, s), "adjoint: 2-D steps");
+    cur ^= 1;
+    return GBS_OK;
+  };
   // one adjoint step lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_t) on state u_t
-  auto step = [&](const char *u) -> gbs_status {
+  auto step = [&](const char *u, bool follows) -> gbs_status {
+    if (blocked) return steps(u, 1, follows);
     if (gradient) {
-      CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s, false),
+      CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s, follows),
          "adjoint: gradient2d step");
-    } else if (g.dim == 2 && sd->nterms <= kMaxCoefGrad) {
-      CK(K.fused2d(g, lam[cur], u, lam[cur ^ 1], hg, part, coef, div, dev_coef_grad != nullptr, s),
-         "adjoint: fused 2-D step");
     } else {
       CK(K.halo(g, lam[cur], hg, coef, div, s), "adjoint: halo");
       if (dev_coef_grad) CK(K.coef(g, lam[cur], u, part, div, s), "adjoint: coefficients");
@@ -1223,8 +1002,12 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
 
   if (!gradient && !dev_coef_grad) {
     // no forward state enters: T transposed steps from lam_T
-    for (int t = d->timestep - 1; t >= 0; --t)
-      if ((st = step(nullptr)) != GBS_OK) return st;
+    for (int left = d->timestep; left > 0;) {
+      const int b = blocked ? degree(left) : 1;
+      st = blocked ? steps(nullptr, b, left < d->timestep) : step(nullptr, false);
+      if (st != GBS_OK) return st;
+      left -= b;
+    }
   } else if (w.revolve) {
     // Each chunk reversed by the binomial schedule over `slots` snapshot
     // planes and two work planes, all on `s`. The halo of every stash plane
@@ -1258,14 +1041,14 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
                                                                          int top) -> gbs_status {
       const int l = b - a, nfree = w.slots - top;
       if (l <= 0) return GBS_OK;
-      if (l == 1) return step(ua);
+      if (l == 1) return step(ua, false);
       if (nfree == 0) {
         for (int t = b - 1; t > a; --t) {
           gbs_status r = advance(ua, work1, t - a);
-          if (r == GBS_OK) r = step(work1);
+          if (r == GBS_OK) r = step(work1, false);
           if (r != GBS_OK) return r;
         }
-        return step(ua);
+        return step(ua, false);
       }
       const int m = revolve_split(l, nfree);
       char *snap = stash + (size_t)top * w.plane_bytes;
@@ -1358,7 +1141,12 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       cudaStreamWaitEvent(s, ready[b], 0);
       // lam_{t+1} -> lam_t for t = t0+c-1 .. t0
       char *buf = stash + (size_t)b * buf_bytes;
-      for (int k = c - 1; k >= 0 && st == GBS_OK; --k) st = step(buf + (size_t)k * w.plane_bytes);
+      for (int k = c - 1; k >= 0 && st == GBS_OK;) {
+        const int bb = blocked ? degree(k + 1) : 1;
+        const char *u = buf + (size_t)k * w.plane_bytes;
+        st = blocked ? steps(u, bb, k < c - 1) : step(u, gradient && k < c - 1);
+        k -= bb;
+      }
       cudaEventRecord(freed[b], s);
     }
     // every piece of s2's work is ordered before s (the last ready event); join anyway

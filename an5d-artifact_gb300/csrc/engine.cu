@@ -256,9 +256,9 @@ int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_war
   const double overlap = 2.0 * br + 2.0;
   double best = 1e300;
   int best_sl = ni;
-  // more blocks than fill the chip 16 times over gain nothing
-  const long long most = std::min<long long>(ni, std::max<long long>(1, 16LL * sms * res * kWarpsPerCta2D / nstrips));
-  for (long long nb = 1; nb <= most; ++nb) {
+  // for every number of CTAs on the busiest SM (up to 16 waves), the most blocks
+  for (long long k = 1; k <= 16LL * res; ++k) {
+    const long long nb = std::max<long long>(1, std::min<long long>(ni, k * sms * kWarpsPerCta2D / nstrips));
     const int sl = (int)((ni + nb - 1) / nb);
     const long long ctas = ((ni + sl - 1) / sl * (long long)nstrips + kWarpsPerCta2D - 1) / kWarpsPerCta2D;
     const long long per_sm = (ctas + sms - 1) / sms;
@@ -269,6 +269,7 @@ int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_war
       best = cost;
       best_sl = sl;
     }
+    if (nb == ni) break;
   }
   return best_sl;
 }

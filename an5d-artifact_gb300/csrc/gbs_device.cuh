@@ -177,6 +177,43 @@ __device__ __forceinline__ void st_vec_global(T *p, const T (&x)[V]) {
 template <typename T>
 __device__ __forceinline__ void st_global(T *p, T v) { __stcg(p, v); }
 
+// Predicated forms, for stores that a few lanes make in straight-line code: as
+// branches they split a row into divergent pieces that cannot be scheduled
+// across.
+__device__ __forceinline__ void st_global_if(float *p, float v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q st.global.cg.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v),
+               "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void st_global_if(double *p, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q st.global.cg.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+               "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void red_add_if(float *p, float v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q red.global.add.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v),
+               "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void red_add_if(double *p, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+               "r"((int)on)
+               : "memory");
+}
+template <int V> __device__ __forceinline__ void st_vec_global_if(float *p, const float (&x)[V], bool on) {
+  static_assert(V == 4, "16-byte vectors only");
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q st.global.cg.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(p),
+      "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "r"((int)on)
+      : "memory");
+}
+template <int V> __device__ __forceinline__ void st_vec_global_if(double *p, const double (&x)[V], bool on) {
+  static_assert(V == 2, "16-byte vectors only");
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q st.global.cg.v2.f64 [%0], {%1, %2};\n\t}" ::"l"(p),
+               "d"(x[0]), "d"(x[1]), "r"((int)on)
+               : "memory");
+}
+
 // ---- lane shuffles -----------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T shfl_up(T v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }

@@ -395,33 +395,24 @@ __device__ __forceinline__ void warp_item2d(const Params2D<T, ST::kTerms> &p, in
       const int pp = pb + ph;
       T x[V];
       ld_ring<PP>(x, my + rd + (unsigned)ph * PP::ROWB);
+      // the lane's columns of an output row; outside the edge strips a lane is
+      // stored whole or not at all
+      auto store = [&](T *d, bool on) GBS_INL {
+        st_vec_global_if<V>(d, x, on && store_all);
+        if constexpr (care != kInterior) {
+#pragma unroll
+          for (int e = 0; e < V; ++e) st_global_if(d + e, x[e], on && !store_all && col0 + e >= cs && col0 + e < ce);
+        }
+      };
       static_for<B>([&](auto LI) GBS_INL {
         constexpr int l = decltype(LI)::value;
         level2d<ST, PP, T, FMA, care, ph>(win[l], up[l], x, pp - (l + 1) * R, fixed, carry, p);
         if constexpr (STASH && l + 1 < B) {
-          const unsigned ql = (unsigned)(pp - (l + 1) * R - i0);
-          if (ql < nout) {
-            T *d = ss + (long long)l * p.stash_stride - (long long)((l + 1) * R) * p.pitch;
-            if (store_all) {
-              st_vec_global<T, V>(d, x);
-            } else if constexpr (care != kInterior) {
-#pragma unroll
-              for (int e = 0; e < V; ++e)
-                if (col0 + e >= cs && col0 + e < ce) st_global(d + e, x[e]);
-            }
-          }
+          store(ss + (long long)l * p.stash_stride - (long long)((l + 1) * R) * p.pitch,
+                (unsigned)(pp - (l + 1) * R - i0) < nout);
         }
       });
-      if ((unsigned)(pp - B * R - i0) < nout) {
-        if (store_all) {
-          st_vec_global<T, V>(st, x);
-        } else if constexpr (care != kInterior) {
-          // outside the edge strips a lane is stored whole or not at all
-#pragma unroll
-          for (int e = 0; e < V; ++e)
-            if (col0 + e >= cs && col0 + e < ce) st_global(st + e, x[e]);
-        }
-      }
+      store(st, (unsigned)(pp - B * R - i0) < nout);
       st += p.pitch;
       if constexpr (STASH) ss += p.pitch;
     });

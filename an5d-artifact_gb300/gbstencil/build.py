@@ -54,8 +54,12 @@ def units():
                              f"-DGBS_PICK=picks_{sid}_{t}_{m}"]))
     for m in (0, 1):  # the batched kernel, exact and FMA mode
         out.append((f"batch_{m}", CSRC / "batch.cu", [f"-DGBS_FMA={m}"]))
+    for sid in range(6):  # the 2-D adjoint steps: star2d1r-4r, box2d1r, box2d2r (adjoint_internal.h)
+        for t, T in (("f", "float"), ("d", "double")):
+            out.append((f"adjoint2d_{sid}_{t}", CSRC / "adjoint2d.cu",
+                        [f"-DGBS_SID={sid}", f"-DGBS_T={T}", f"-DGBS_PICK=adj2d_picks_{sid}_{t}"]))
     for src in sorted(CSRC.glob("*.cu")):
-        if src.name not in ("inst.cu", "batch.cu"):
+        if src.name not in ("inst.cu", "batch.cu", "adjoint2d.cu"):
             out.append((src.stem, src, []))
     return out
 
@@ -107,7 +111,7 @@ def build(jobs: int | None = None, verbose: bool = False, regcap: int = 0) -> Pa
         us = [(n, s, f + [f"-DGBS_REGCAP={regcap}"]) for n, s, f in us]
     # the slowest units first: the batched kernels (every 2-D stencil in one
     # unit), then the big-radius 3-D boxes
-    us.sort(key=lambda u: 0 if u[0].startswith("batch_") else (1 if "picks_1" in u[0] else 2))
+    us.sort(key=lambda u: 0 if u[0].startswith(("batch_", "adjoint")) else (1 if "picks_1" in u[0] else 2))
     changed = False
     with ThreadPoolExecutor(max_workers=jobs) as ex:
         for name, did, log in ex.map(lambda u: compile_unit(u, verbose, build_dir), us):
