@@ -514,7 +514,10 @@ Workspace workspace_of(const gbs_desc *d, const Layout &L, int C, int slots) {
   w.off_stash = w.off_cp + (size_t)w.ncp * w.plane_bytes;
   w.off_lam = w.off_stash + (size_t)(w.revolve ? w.slots + 2 : 2 * C) * w.plane_bytes;
   w.off_hg = w.off_lam + 2 * w.plane_bytes;
-  w.off_part = w.off_hg + w.plane_bytes;
+  // gradient2d: two planes more than its step needs, so that a workspace or a
+  // budget holds as many checkpoints and slots as it did when that step kept
+  // per-cell values between two passes
+  w.off_part = w.off_hg + (s->kind == 1 ? 3 : 1) * w.plane_bytes;
   w.total = w.off_part + (size_t)w.nblocks * w.nt * sizeof(double) + 256;
   return w;
 }

@@ -12,8 +12,9 @@
 // allocation, reaching the item's `need`). The order (by time block) makes
 // this deadlock-free: every item an item waits on was taken earlier by a
 // running CTA that never waits on a later item. Waits are bounded (the
-// error word is set and the CTA stops). The layered schedule runs the same
-// items as one kernel node per time block instead, with no waits.
+// error word is set and the CTA stops). The layered schedule runs its items
+// as chains of kernel nodes instead, one chain per stencil and a node per time
+// block, with no waits on the device (batch_family_kernel, kernel2d.cuh).
 //
 // Memory ordering: a finishing item's lanes fence their stores, then lane 0
 // increments its block's counter; a starting item's lane 0 reads the
@@ -37,41 +38,15 @@
 #endif
 
 namespace gbs {
-namespace batchdetail {
-constexpr int kMaxTerms = 81;
-
-struct GridDev {
-  float *base;          // two-plane buffer (engine layout)
-  long long pitch, plane;
-  int d0, d1, shift, sid;
-  int sl, nblocks;
-  // completion counters of the grid: done[cbase .. cbase + ccount); one per
-  // stream block (an item waits for its own block and the two beside it),
-  // or one for the whole grid (an item waits for every earlier item of it)
-  int cbase, ccount;
-  float coef[kMaxTerms];
-  float div, rdiv, eps;
-  int divmode;
-};
-
-struct Item {
-  int grid, k, b, strip, blk, need, pad0, pad1;
-};
-}  // namespace batchdetail
-using batchdetail::GridDev;
-using batchdetail::Item;
+using GridDev = BatchGridDev;
+using Item = BatchItem;
 
 namespace {
 constexpr bool kFma = GBS_FMA != 0;
 constexpr int kWpc = kWpc2D;
-// CTAs per SM the batched kernels are built for. The layered kernel takes 4
-// (at most 128 registers a thread, 16 warps an SM; every variant but
-// star2d3r at degree 2 fits without spilling): 2.92x the per-grid launches
-// on the 512-grid mix against 2.76x at 3 CTAs (168 registers, of which the
-// heaviest variants use 154-164 and so set them for all). The persistent
-// kernel keeps 3: at 4 its warps stalled more on instruction fetch (more
-// variants resident per SM) and it was 1% slower.
-constexpr int kLayerCtas = 4, kPersistentCtas = 3;
+// CTAs per SM the persistent kernel is built for: at 4 its warps stalled more
+// on instruction fetch (more variants resident per SM) and it was 1% slower.
+constexpr int kPersistentCtas = 3;
 
 // The stencils a batch may mix and the fused degree used for each (the full
 // blocks; remainders run at degree 1). Measured on the 512-grid mix
@@ -101,10 +76,6 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   return v;
 }
 
-// bytes of the per-warp shared-memory slot that holds an item's parameters
-constexpr int kParamSlot = 512;
-static_assert(sizeof(Params2D<float, batchdetail::kMaxTerms>) <= kParamSlot, "parameter slot too small");
-
 // One (stencil, degree) variant per function, not inlined: each variant gets
 // its own register allocation (inlining all of them into the dispatcher
 // forces a local-memory frame onto every variant's loop) and the call costs
@@ -119,23 +90,7 @@ __device__ __noinline__ void run_item(const GridDev *gp, int k, int strip, int b
   auto &p = *reinterpret_cast<Params2D<float, S::kTerms> *>(slot);
   const int lane = threadIdx.x & 31;
   for (int t = lane; t < S::kTerms; t += 32) p.coef[t] = g.coef[t];
-  if (lane == 0) {
-    p.src = g.base + (long long)(k % 2) * g.plane;
-    p.dst = g.base + (long long)((k + 1) % 2) * g.plane;
-    p.pitch = g.pitch;
-    p.d0 = g.d0;
-    p.d1 = g.d1;
-    p.shift = g.shift;
-    p.nstrips = 0;
-    p.nblocks = g.nblocks;
-    p.sl = g.sl;
-    p.div = g.div;
-    p.rdiv = g.rdiv;
-    p.eps = g.eps;
-    p.divmode = g.divmode;
-    p.stash = nullptr;
-    p.stash_stride = 0;
-  }
+  if (lane == 0) batch_params<S>(p, g, k, g.sl);
   __syncwarp();
   if constexpr (S::kTerms <= 25) {
     // small parameter sets ride in registers for the whole item
@@ -230,14 +185,13 @@ __device__ __forceinline__ bool persistent_item(const Args &a, unsigned idx, uns
 }
 
 // Persistent: each CTA takes groups of kWpc consecutive items from an
-// atomic counter, warp w running item group * kWpc + w, the way the layered
-// schedule's CTAs run consecutive items. Neighbouring items are the same
-// stencil and degree (consecutive strips of one stream block), so the CTAs
-// resident on an SM mostly run one kernel variant and share its code in the
-// instruction cache; warps that took items one at a time mixed variants on
-// every SM and stalled on instruction fetch. Groups are taken in order and
-// an item waits only on earlier items, whose groups were taken by running
-// CTAs: progress does not need every CTA resident.
+// atomic counter, warp w running item group * kWpc + w. Neighbouring items
+// are the same stencil and degree (consecutive strips of one stream block),
+// so the CTAs resident on an SM mostly run one kernel variant and share its
+// code in the instruction cache; warps that took items one at a time mixed
+// variants on every SM and stalled on instruction fetch. Groups are taken in
+// order and an item waits only on earlier items, whose groups were taken by
+// running CTAs: progress does not need every CTA resident.
 __global__ void __launch_bounds__(kWpc * 32, kPersistentCtas) batch2d_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ unsigned s_group;
@@ -257,19 +211,6 @@ __global__ void __launch_bounds__(kWpc * 32, kPersistentCtas) batch2d_kernel(con
         (threadIdx.x & 31) == 0)
       s_stop = 1;
   }
-}
-
-// One time block of every grid: warp w runs item first + w. Kernel
-// boundaries order the blocks, so nothing here waits.
-__global__ void __launch_bounds__(kWpc * 32, kLayerCtas) batch_layer_kernel(const __grid_constant__ Args a, int first,
-                                                                   int count) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const long long gw = (long long)blockIdx.x * kWpc + (threadIdx.x >> 5);
-  if (gw >= count) return;
-  unsigned char *ring = smem_raw + (size_t)(threadIdx.x >> 5) * kRing;
-  unsigned char *slot = smem_raw + (size_t)kWpc * kRing + (size_t)(threadIdx.x >> 5) * kParamSlot;
-  const Item it = a.items[first + gw];
-  dispatch(a.grids[it.grid], it, ring, slot);
 }
 
 // ---------------------------------------------------------------------------
@@ -303,14 +244,55 @@ std::vector<int> batch_blocks(int T, int bs) {
   for (int i = 0; i < r; ++i) out.push_back(1);
   return out;
 }
+
+// degree of the layered schedule's full blocks
+int layered_degree(int sid) {
+  const Picks &p = batch_picks(sid, kFma ? 1 : 0);
+  int b = 0;
+  while (b < kBatchMaxB && p.lb[b + 1]) ++b;
+  return b;
+}
+
+// Time blocks of T steps for the layered schedule: what is left over by full
+// blocks of bs steps first, so that the grids of a stencil soon run at the
+// same degree, then the full blocks; as many blocks as T has parity (launch k
+// reads plane k%2), for which the rest, or a full block, is split in two.
+// For odd T the last block has the steps that batch_blocks gives it: the plane
+// without the result keeps the state before it, from which a run of odd T that
+// is repeated starts, under every schedule.
+std::vector<int> layered_blocks(int T, int bs, int persistent_bs) {
+  std::vector<int> out;
+  if (T <= 0 || bs < 1) return out;
+  const int last = T % 2 ? batch_blocks(T, persistent_bs).back() : 0;
+  T -= last;  // an even rest
+  int full = T / bs;
+  const int rest = T - full * bs;
+  auto halves = [&](int x) {
+    out.push_back((x + 1) / 2);
+    out.push_back(x / 2);
+  };
+  if (T == 0) {
+  } else if ((full + (rest > 0) - T) % 2 == 0) {
+    if (rest > 0) out.push_back(rest);
+  } else if (rest >= 2) {
+    halves(rest);
+  } else {  // a full block goes, and one or three blocks take its steps
+    --full;
+    halves(bs);
+    if (rest > 0) out.push_back(rest);
+  }
+  out.insert(out.end(), full, bs);
+  if (last > 0) out.push_back(last);
+  return out;
+}
 }  // namespace
 }  // namespace gbs
 
 using namespace gbs;
 
 struct gbs_batch {
-  gbs::batchdetail::GridDev *d_grids = nullptr;
-  gbs::batchdetail::Item *d_items = nullptr;
+  gbs::GridDev *d_grids = nullptr;
+  gbs::Item *d_items = nullptr;
   unsigned *d_counters = nullptr;  // [0] next, [1..] done per stream block of every grid
   int ncounters = 0;
   int ngrids = 0, nitems = 0, ctas = 0;
@@ -363,12 +345,11 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
     x.shift = (int)L.shift;
     x.sid = bg.stencil;
     const int ni = L.dims[0] - 2 * s->rad;
-    // stream blocks long enough to amortise an item's start (dependency
-    // check, first copies), short enough that a time block's items finish
-    // together. Measured on the 512-grid mix: layered 64 / 96 / 128 / 256
-    // rows gave 3.00 / 3.01 / 2.98 / 2.47x the per-grid launches, persistent
-    // 2.65x at 64 rows and 2.71x at 128.
-    x.sl = std::min(ni, mode == GBS_BATCH_LAYERED ? 96 : 128);
+    // persistent: stream blocks long enough to amortise an item's start
+    // (dependency check, first copies), short enough that a time block's
+    // items finish together (512-grid mix: 2.65x the per-grid launches at 64
+    // rows, 2.71x at 128); the layered schedule chooses per launch (below)
+    x.sl = std::min(ni, 128);
     x.nblocks = (ni + x.sl - 1) / x.sl;
     const double div = bg.divisor != 0.0 ? bg.divisor : (double)s->divisor;
     const bool fold = kFma && s->divisor;
@@ -382,10 +363,15 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
     x.rdiv = div_reciprocal<float>(div);
     x.eps = (float)s->eps;
     x.divmode = !s->divisor || fold ? 0 : (div_proven_exact(div) ? 2 : 1);
-    blocks[g] = batch_blocks(bg.timestep, family_degree(bg.stencil));
+    blocks[g] = mode == GBS_BATCH_LAYERED ? layered_blocks(bg.timestep, layered_degree(bg.stencil), family_degree(bg.stencil))
+                                          : batch_blocks(bg.timestep, family_degree(bg.stencil));
+    if (bg.timestep > 0 && blocks[g].empty())
+      return fail(GBS_ERR_UNSUPPORTED, "batch grid %d: no batched kernels built for %s", g, s->name);
     cells += (long long)bg.n[0] * bg.n[1] * bg.timestep;
     // validate every strip window of every degree used
-    for (int b : blocks[g]) {
+    for (size_t k = 0; k < blocks[g].size(); ++k) {
+      const int b = blocks[g][k];
+      if (k > 0 && b == blocks[g][k - 1]) continue;
       Geometry2D geo = geometry2d(L, b, x.sl, 0);
       gbs_status st = validate2d(L, geo);
       if (st != GBS_OK) return st;
@@ -410,22 +396,59 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
   std::vector<int> done_before(ngrids, 0);
   size_t kmax = 0;
   for (auto &b : blocks) kmax = std::max(kmax, b.size());
-  std::vector<int> layer_start;
-  for (size_t k = 0; k < kmax; ++k)
-  for (int sid = 0; sid < GBS_NUM_STENCILS; ++sid) {
-    if (sid == 0) layer_start.push_back((int)items.size());
+  if (mode == GBS_BATCH_PERSISTENT)
+    for (size_t k = 0; k < kmax; ++k)
+      for (int sid = 0; sid < GBS_NUM_STENCILS; ++sid)
+        for (int g = 0; g < ngrids; ++g) {
+          if (grids[g].stencil != sid || k >= blocks[g].size()) continue;
+          const int b = blocks[g][k];
+          const int rad = stencil_def(sid)->rad;
+          const int wout = wout2d(rad, b, 4);
+          const int nstrips = (gd[g].d1 - 2 * rad + wout - 1) / wout;
+          for (int blk = 0; blk < gd[g].nblocks; ++blk)
+            for (int st = 0; st < nstrips; ++st)
+              items.push_back(Item{g, (int)k, b, st, blk, done_before[g], gd[g].sl, 0});
+          done_before[g] += nstrips;
+        }
+  // Layered: per stencil a chain of launches, one per time block and degree
+  // (chains of different stencils are independent, and grids of one stencil
+  // meet in a launch only where they are at the same degree). Rows per item: a
+  // chain takes about its number of launches times its items' cost, so the
+  // items of a long chain are the shorter ones, such that all chains end
+  // together while their items fill the chip once (kFill warps): with few
+  // grids, long items leave the chip idle behind the longest chain. Within
+  // [2*b*r, 128] rows, for the overlap's sake and for large batches.
+  struct Group {
+    int sid, b, first, count;
+  };
+  std::vector<Group> groups;
+  if (mode == GBS_BATCH_LAYERED) {
+    constexpr double kFill = 152 * 12;
+    double work = 0.0;
+    std::vector<size_t> chain(GBS_NUM_STENCILS, 0);
+    auto strips = [&](int g, int b) {
+      const int rad = stencil_def(grids[g].stencil)->rad, wout = wout2d(rad, b, 4);
+      return (gd[g].d1 - 2 * rad + wout - 1) / wout;
+    };
+    auto row_cost = [&](int g, int b) { return (double)batch_picks(grids[g].stencil, kFma ? 1 : 0).row_cost[b]; };
     for (int g = 0; g < ngrids; ++g) {
-      if (grids[g].stencil != sid || k >= blocks[g].size()) continue;
-      const int b = blocks[g][k];
-      const gbs_stencil_def_t *s = stencil_def(grids[g].stencil);
-      const int wout = wout2d(s->rad, b, 4);
-      const int nj = gd[g].d1 - 2 * s->rad;
-      const int nstrips = (nj + wout - 1) / wout;
-      const int need = done_before[g];
-      for (int blk = 0; blk < gd[g].nblocks; ++blk)
-        for (int st = 0; st < nstrips; ++st) items.push_back(Item{g, (int)k, b, st, blk, need, 0, 0});
-      done_before[g] += nstrips;
+      for (int b : blocks[g]) work += row_cost(g, b) * strips(g, b) * grids[g].n[0];
+      chain[grids[g].stencil] = std::max(chain[grids[g].stencil], blocks[g].size());
     }
+    for (int sid = 0; sid < GBS_NUM_STENCILS; ++sid)
+      for (size_t k = 0; k < kmax; ++k)
+        for (int b = kBatchMaxB; b >= 1; --b) {
+          const int first = (int)items.size();
+          for (int g = 0; g < ngrids; ++g) {
+            if (grids[g].stencil != sid || k >= blocks[g].size() || blocks[g][k] != b) continue;
+            const int br = b * stencil_def(sid)->rad, ni = grids[g].n[0];
+            const double want = work / (kFill * (double)chain[sid] * row_cost(g, b)) - 2.0 * br;
+            const int sl = std::min(ni, std::max(std::max(4, 2 * br), (int)std::min(128.0, want)));
+            for (int blk = 0; blk < (ni + sl - 1) / sl; ++blk)
+              for (int st = 0; st < strips(g, b); ++st) items.push_back(Item{g, (int)k, b, st, blk, 0, sl, 0});
+          }
+          if ((int)items.size() > first) groups.push_back(Group{sid, b, first, (int)items.size() - first});
+        }
   }
   auto *h = new gbs_batch();
   h->ngrids = ngrids;
@@ -474,17 +497,51 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
     gbs_batch_destroy(h);
     return cuda_fail(e, "batch: stream");
   }
-  layer_start.push_back((int)items.size());
   h->mode = mode;
+  cudaStream_t side[GBS_NUM_STENCILS] = {};
+  cudaEvent_t fork = nullptr, join[GBS_NUM_STENCILS] = {};
+  if (mode == GBS_BATCH_LAYERED) {
+    e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    for (const Group &q : groups) {
+      if (e != cudaSuccess || side[q.sid]) continue;
+      e = cudaStreamCreateWithFlags(&side[q.sid], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join[q.sid], cudaEventDisableTiming);
+    }
+  }
+  auto release = [&]() {
+    for (int k = 0; k < GBS_NUM_STENCILS; ++k) {
+      if (join[k]) cudaEventDestroy(join[k]);
+      if (side[k]) cudaStreamDestroy(side[k]);
+    }
+    if (fork) cudaEventDestroy(fork);
+    cudaStreamDestroy(cs);
+  };
+  if (e != cudaSuccess) {
+    release();
+    gbs_batch_destroy(h);
+    return cuda_fail(e, "batch: streams");
+  }
+  cudaError_t launch_error = cudaSuccess;
   e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     if (mode == GBS_BATCH_LAYERED) {
-      for (size_t k = 0; k + 1 < layer_start.size(); ++k) {
-        const int first = layer_start[k], count = layer_start[k + 1] - first;
-        if (count <= 0) continue;
-        batch_layer_kernel<<<(count + kWpc - 1) / kWpc, kWpc * 32, h->smem, cs>>>(a, first, count);
+      cudaError_t le = cudaEventRecord(fork, cs);
+      for (int k = 0; k < GBS_NUM_STENCILS; ++k)
+        if (side[k] && le == cudaSuccess) le = cudaStreamWaitEvent(side[k], fork, 0);
+      int prev = -1;
+      for (const Group &q : groups) {
+        if (le != cudaSuccess) break;
+        le = batch_picks(q.sid, kFma ? 1 : 0)
+                 .lb[q.b](h->d_grids, h->d_items, q.first, q.count, side[q.sid], q.sid == prev);
+        prev = q.sid;
         ++h->kernels;
       }
+      for (int k = 0; k < GBS_NUM_STENCILS; ++k) {  // join even after a failure, so that the capture can end
+        if (!side[k]) continue;
+        cudaEventRecord(join[k], side[k]);
+        cudaStreamWaitEvent(cs, join[k], 0);
+      }
+      launch_error = le;
     } else {
       cudaMemsetAsync(h->d_counters, 0, sizeof(unsigned) * (ncounters + 1), cs);
       batch2d_kernel<<<h->ctas, kWpc * 32, h->smem, cs>>>(a);
@@ -492,8 +549,9 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
     }
     e = cudaStreamEndCapture(cs, &h->graph);
   }
+  if (launch_error != cudaSuccess) e = launch_error;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&h->exec, h->graph, 0);
-  cudaStreamDestroy(cs);
+  release();
   if (e != cudaSuccess) {
     gbs_batch_destroy(h);
     return cuda_fail(e, "batch: graph capture");
@@ -630,7 +688,7 @@ gbs_status run(const gbs_batch_grid *grids, int ngrids, cudaStream_t stream) {
                       "(use gbs_batch_plan for larger batches)",
                       kMaxItems);
         for (int blk = 0; blk < h_grids[g].nblocks; ++blk)
-          for (int st = 0; st < nstrips; ++st) h_items[nitems++] = Item{g, k, b, st, blk, done_before[g], 0, 0};
+          for (int st = 0; st < nstrips; ++st) h_items[nitems++] = Item{g, k, b, st, blk, done_before[g], h_grids[g].sl, 0};
         done_before[g] += count;
       }
   if (nitems == 0) return GBS_OK;
@@ -747,7 +805,6 @@ gbs_status build_streams(const gbs_batch_grid *grids, int ngrids, int dtype, int
     // GBS_BATCH_SHARE=1: stream length for this grid's share of one wave
     // (default: the single-grid choice, one whole wave per kernel, which
     // measured faster on GB300: 254 vs 220 GCells/s at 16 branches)
-    d.bt = pi.bt;
     const char *share_env = std::getenv("GBS_BATCH_SHARE");
     if (s->dim == 2 && d.sl == 0 && share_env && share_env[0] == '1') {
       const Layout L = make_layout(&d);

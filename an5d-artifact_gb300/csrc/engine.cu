@@ -73,6 +73,8 @@ static const Picks &picks(int sid, int dtype, int fma) {
   return table[sid][dtype][fma];
 }
 
+const Picks &batch_picks(int sid, int fma) { return picks(sid, GBS_F32, fma); }
+
 int max_bt(int sid, int dtype, int fma) { return picks(sid, dtype, fma).maxb; }
 
 // ---------------------------------------------------------------------------
@@ -211,6 +213,27 @@ std::vector<int> split_steps(int T, int bt) {
   if ((n - T) % 2 != 0) ++n;
   const int q = T / n, rem = T % n;
   for (int j = 0; j < n; ++j) out.push_back(q + (j < rem ? 1 : 0));
+  return out;
+}
+
+static int default_bt(const gbs_desc *d);
+std::vector<int> loop_steps(const gbs_desc *d, int bt) {
+  const int T = d->timestep;
+  if (T % 2 == 0 || d->bt > 0) return split_steps(T, bt);
+  int lb = tuned_last(d);
+  if (lb == 0) lb = default_bt(d);
+  const int last = split_steps(T, lb).back();
+  // an even number of launches for the rest (at least 2 T/3 steps, or none)
+  std::vector<int> out;
+  const int rest = T - last;
+  if (rest > 0) {
+    int n = (rest + bt - 1) / bt;
+    n += n % 2;
+    if (n > rest) n -= 2;  // degree 1 and an odd rest: one launch takes two steps (the last takes as many)
+    const int q = rest / n, rem = rest % n;
+    for (int j = 0; j < n; ++j) out.push_back(q + (j < rem ? 1 : 0));
+  }
+  out.push_back(last);
   return out;
 }
 
@@ -511,7 +534,7 @@ gbs_status run_loop(const gbs_desc *d, const Layout &L, void *dev_A, cudaStream_
   const double eps = d->eps != 0.0 ? d->eps : (double)s->eps;
   if (s->divisor && div == 0.0) return fail(GBS_ERR_INVALID, "divisor must be nonzero");
 
-  const std::vector<int> steps = split_steps(d->timestep, bt);
+  const std::vector<int> steps = loop_steps(d, bt);
   char *base = static_cast<char *>(dev_A);
   const size_t plane_bytes = (size_t)L.plane * L.esize;
   BlockPlan plan;  // the steps come in one run of each degree
@@ -681,7 +704,7 @@ gbs_status gbs_plan(const gbs_desc *d, gbs_plan_info *out) {
   if (bt > mx) return fail(GBS_ERR_UNSUPPORTED, "bt=%d exceeds the largest fused degree built (%d)", bt, mx);
   std::memset(out, 0, sizeof *out);
   out->bt = bt;
-  out->launches = (int)split_steps(d->timestep, bt).size();
+  out->launches = (int)loop_steps(d, bt).size();
   if (s->dim == 2) {
     Geometry2D g = geometry2d(L, bt, sl, resident_warps_2d(d->stencil, d->dtype, fma, bt));
     st = validate2d(L, g);

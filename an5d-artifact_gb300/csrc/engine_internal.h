@@ -51,6 +51,9 @@ const gbs_stencil_def_t *stencil_def(int sid);
 gbs_status check_desc(const gbs_desc *d);
 Layout make_layout(const gbs_desc *d);
 std::vector<int> split_steps(int T, int bt);
+// The launches of d's time loop at degree bt: split_steps, but for odd T the
+// last launch takes the steps that the degree of tuned_last would give it.
+std::vector<int> loop_steps(const gbs_desc *d, int bt);
 // resident_warps: warps the GPU holds at once for this kernel (0 = unknown)
 // rows per stream block of a 2-D launch of nstrips strips over ni rows whose
 // blocks overlap by br rows at each end
@@ -86,9 +89,14 @@ gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, 
 // be null)
 gbs_status launch_block_stash(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                               int b, const void *src, void *dst, void *stash, cudaStream_t stream, int *err);
+// the layered batched launchers of a stencil (Picks::lb) and their row costs
+const Picks &batch_picks(int sid, int fma);
 int max_bt(int sid, int dtype, int fma);
 // the tuning table's (bt, sl) for d's stencil, dtype, mode and size class
 bool tuned_lookup(const gbs_desc *d, int *bt, int *sl, int *bs1 = nullptr);
+// the degree that fixes the last launch's steps of a loop of odd T for d's
+// stencil, dtype, mode and size class (0: no entry); see loop_steps
+int tuned_last(const gbs_desc *d);
 bool div_proven_exact(double d);
 
 }  // namespace gbs

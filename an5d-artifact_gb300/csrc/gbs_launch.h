@@ -75,8 +75,36 @@ constexpr int kMaxStashB = 4;
 // warps (tile rows = warps x rows per warp)
 constexpr int kVar3 = 2;
 constexpr int kTileWarps[kVar3] = {16, 8};
+// One grid of a batched launch, in device memory (float grids).
+constexpr int kBatchMaxTerms = 81;
+struct BatchGridDev {
+  float *base;          // two-plane buffer (engine layout)
+  long long pitch, plane;
+  int d0, d1, shift, sid;
+  int sl, nblocks;      // rows per stream block (persistent schedule) and their number
+  // completion counters of the grid: done[cbase .. cbase + ccount); one per
+  // stream block (an item waits for its own block and the two beside it),
+  // or one for the whole grid (an item waits for every earlier item of it)
+  int cbase, ccount;
+  float coef[kBatchMaxTerms];
+  float div, rdiv, eps;
+  int divmode;
+};
+// One work item: strip `strip`, stream block `blk` (of sl rows) of time block
+// k (b steps) of a grid. need: items of its counters in earlier time blocks.
+struct BatchItem {
+  int grid, k, b, strip, blk, need, sl, pad;
+};
+// Launches items [first, first + count), all of one stencil and degree.
+using BatchFn = cudaError_t (*)(const BatchGridDev *grids, const BatchItem *items, int first, int count,
+                                cudaStream_t stream, bool pdl);
+// largest degree of the layered batched kernels
+constexpr int kBatchMaxB = 6;
+
 struct Picks {
   int maxb;
+  BatchFn lb[kBatchMaxB + 1];     // layered batched launchers (2-D float; else null)
+  int row_cost[kBatchMaxB + 1];   // warp instructions of one row of theirs, about
   Launch2DFn l2[kMaxB + 1];
   Launch2DFn l2s[kMaxB + 1];    // stash-mode 2-D launchers (FMA mode, low degrees; else null)
   Occupancy2DFn o2[kMaxB + 1];

@@ -79,12 +79,26 @@ template <int B, int V> void add_variant3(Picks &p) {
   }
 }
 
+// Degrees of the layered batched kernels: a grid takes blocks of the largest
+// and at most two smaller ones for the rest.
+constexpr int batch_class() {
+  if (S::kDim != 2) return 0;
+  const int m = S::kKind == KIND_GRADIENT ? 1 : S::kRad == 1 ? 6 : S::kRad == 2 ? (S::kTerms > 13 ? 2 : 4)
+                : S::kRad == 3 ? (S::kAssoc ? 1 : 2) : (S::kAssoc ? 1 : 2);
+  return m < max_class() ? m : max_class();
+}
+static_assert(batch_class() <= kBatchMaxB, "batched degrees");
+
 template <int B> void add(Picks &p) {
   if constexpr (B <= max_class()) {
     if constexpr (S::kDim == 2) {
       p.l2[B] = &launch2d<S, T, B, kFma>;
       p.o2[B] = &occupancy2d<S, T, B, kFma>;
       if constexpr (kFma && B >= 2 && B <= kMaxStashB) p.l2s[B] = &launch2d<S, T, B, kFma, true>;
+      if constexpr (sizeof(T) == 4 && B <= batch_class()) {
+        p.lb[B] = &batch_launch<S, B, kFma>;
+        p.row_cost[B] = Pipe2D<S, T, B, kFma>::ROW_INSTR;
+      }
     } else {
       add_variant3<B, 0>(p);
       if constexpr (use_tile3d<S, kFma>()) add_variant3<B, 1>(p);

@@ -515,4 +515,76 @@ cudaError_t launch2d(const Launch2D &a, cudaStream_t stream) {
   return launch_kernel(kern, (unsigned)grid, kWpc2D * 32, smem, stream, a.pdl, p);
 }
 
+// Parameters of one item, from its grid's table entry into p (coefficients by
+// the whole warp; every lane must call it, and p is either every lane's own or
+// shared by the warp).
+template <class ST>
+__device__ __forceinline__ void batch_params(Params2D<float, ST::kTerms> &p, const BatchGridDev &g, int k, int sl) {
+  p.src = g.base + (long long)(k % 2) * g.plane;
+  p.dst = g.base + (long long)((k + 1) % 2) * g.plane;
+  p.pitch = g.pitch;
+  p.d0 = g.d0;
+  p.d1 = g.d1;
+  p.shift = g.shift;
+  p.nstrips = 0;
+  p.nblocks = 0;
+  p.sl = sl;
+  p.div = g.div;
+  p.rdiv = g.rdiv;
+  p.eps = g.eps;
+  p.divmode = g.divmode;
+  p.stash = nullptr;
+  p.stash_stride = 0;
+}
+// bytes of the per-warp shared-memory slot that holds an item's parameters
+// where they do not fit in registers
+constexpr int kParamSlot = 512;
+static_assert(sizeof(Params2D<float, kBatchMaxTerms>) <= kParamSlot, "parameter slot too small");
+
+// Layered batched schedule: one time block of the grids of one stencil at one
+// degree, warp w running item first + w. One kernel per (stencil, degree), so
+// that each gets its own registers and a layer's launches of different
+// stencils need not wait for each other; one kernel that dispatched on the
+// stencil ran every variant at 128 registers and each layer as long as its
+// slowest item: 48 grids of 128..2048 cells a side, up to 128 steps,
+// 9.0 ms -> 4.1 (GB300); the 512-grid mix of the benchmark 370 -> 718 GCells/s.
+template <class ST, int B, bool FMA>
+__global__ void __launch_bounds__(kWpc2D * 32)
+    batch_family_kernel(const BatchGridDev *__restrict__ grids, const BatchItem *__restrict__ items, int count) {
+  constexpr bool SLOT = ST::kTerms > 25;  // more coefficients than registers to spare
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int w = threadIdx.x >> 5;
+  const long long gw = (long long)blockIdx.x * kWpc2D + w;
+  const bool busy = gw < count;
+  const BatchItem it = busy ? items[gw] : BatchItem{};  // the tables do not change: read ahead of the wait
+  const BatchGridDev &g = grids[it.grid];
+  unsigned char *ring = smem_raw + (size_t)w * Pipe2D<ST, float, B, FMA>::RING;
+  if constexpr (SLOT) {
+    auto &p = *reinterpret_cast<Params2D<float, ST::kTerms> *>(
+        smem_raw + (size_t)kWpc2D * Pipe2D<ST, float, B, FMA>::RING + (size_t)w * kParamSlot);
+    for (int t = threadIdx.x & 31; t < ST::kTerms; t += 32) p.coef[t] = g.coef[t];
+    if ((threadIdx.x & 31) == 0) batch_params<ST>(p, g, it.k, it.sl);
+    __syncwarp();
+    wait_for_previous();
+    if (busy) warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
+  } else {
+    Params2D<float, ST::kTerms> p;
+    batch_params<ST>(p, g, it.k, it.sl);
+#pragma unroll
+    for (int t = 0; t < ST::kTerms; ++t) p.coef[t] = g.coef[t];
+    wait_for_previous();
+    if (busy) warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
+  }
+}
+
+template <class ST, int B, bool FMA>
+cudaError_t batch_launch(const BatchGridDev *grids, const BatchItem *items, int first, int count, cudaStream_t stream,
+                         bool pdl) {
+  constexpr size_t smem = smem_bytes2d<ST, float, B, FMA>() + (ST::kTerms > 25 ? kWpc2D * kParamSlot : 0);
+  auto kern = batch_family_kernel<ST, B, FMA>;
+  if (const cudaError_t e = allow_smem2d(kern, smem); e != cudaSuccess) return e;
+  return launch_kernel(kern, (unsigned)((count + kWpc2D - 1) / kWpc2D), kWpc2D * 32, smem, stream, pdl, grids,
+                       items + first, count);
+}
+
 }  // namespace gbs

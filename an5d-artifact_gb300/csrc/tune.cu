@@ -45,6 +45,13 @@ struct Entry {
 
 std::mutex g_mu;
 std::vector<Entry> g_table;
+// The degree that fixes the steps of a time loop's last launch where T is odd
+// (see loop_steps): the plane without the result keeps the state before that
+// launch, and a loop of odd T that is run again starts from it, so a new
+// measurement of the same machine does not change it. Every entry recorded
+// counts for both tables; a line of mode "fma_last" or "exact_last" for this
+// one alone (bt 0: as if the size class had no entry).
+std::vector<Entry> g_last;
 bool g_env_loaded = false;
 
 int size_class(const gbs_desc *d) {
@@ -54,20 +61,33 @@ int size_class(const gbs_desc *d) {
   return cells >= 1.0 ? (int)std::floor(std::log2(cells)) : 0;
 }
 
+void record_in(std::vector<Entry> &t, const Entry &e) {
+  auto it = std::find_if(t.begin(), t.end(), [&](const Entry &x) {
+    return x.sid == e.sid && x.dtype == e.dtype && x.fma == e.fma && x.cls == e.cls;
+  });
+  if (it != t.end()) *it = e;
+  else t.push_back(e);
+}
+void record_locked(const Entry &e) {
+  record_in(g_table, e);
+  record_in(g_last, e);
+}
+
 gbs_status load_locked(const char *path) {
   FILE *f = std::fopen(path, "r");
   if (!f) return fail(GBS_ERR_INVALID, "cannot open tuning table %s", path);
   std::vector<Entry> add;
+  std::vector<bool> last;
   char line[512];
   int lineno = 0;
   while (std::fgets(line, sizeof line, f)) {
     ++lineno;
     char *hash = std::strchr(line, '#');
     if (hash) *hash = 0;
-    char name[64], dt[8], mode[8];
+    char name[64], dt[8], mode[16];
     Entry e{};
     double f7 = 0.0, f8 = 0.0;
-    const int k = std::sscanf(line, "%63s %7s %7s %d %d %d %lf %lf", name, dt, mode, &e.cls, &e.bt, &e.sl, &f7, &f8);
+    const int k = std::sscanf(line, "%63s %7s %15s %d %d %d %lf %lf", name, dt, mode, &e.cls, &e.bt, &e.sl, &f7, &f8);
     if (k <= 0) continue;
     if (k == 7) {
       e.ms = f7;
@@ -80,20 +100,20 @@ gbs_status load_locked(const char *path) {
     }
     e.sid = gbs_stencil_id(name);
     e.dtype = !std::strcmp(dt, "f32") ? GBS_F32 : !std::strcmp(dt, "f64") ? GBS_F64 : -1;
-    e.fma = !std::strcmp(mode, "fma") ? 1 : !std::strcmp(mode, "exact") ? 0 : -1;
-    if (e.sid < 0 || e.dtype < 0 || e.fma < 0 || e.bt < 1 || e.sl < 0) {
+    const bool is_last = !std::strcmp(mode, "fma_last") || !std::strcmp(mode, "exact_last");
+    e.fma = !std::strncmp(mode, "fma", 3) && (is_last || !mode[3]) ? 1
+            : !std::strncmp(mode, "exact", 5) && (is_last || !mode[5]) ? 0 : -1;
+    if (e.sid < 0 || e.dtype < 0 || e.fma < 0 || e.bt < (is_last ? 0 : 1) || e.sl < 0) {
       std::fclose(f);
       return fail(GBS_ERR_INVALID, "%s:%d: bad entry", path, lineno);
     }
     add.push_back(e);
+    last.push_back(is_last);
   }
   std::fclose(f);
-  for (const Entry &e : add) {
-    auto it = std::find_if(g_table.begin(), g_table.end(), [&](const Entry &x) {
-      return x.sid == e.sid && x.dtype == e.dtype && x.fma == e.fma && x.cls == e.cls;
-    });
-    if (it != g_table.end()) *it = e;
-    else g_table.push_back(e);
+  for (size_t i = 0; i < add.size(); ++i) {
+    if (last[i]) record_in(g_last, add[i]);
+    else record_locked(add[i]);
   }
   return GBS_OK;
 }
@@ -104,14 +124,6 @@ void env_load_locked() {
   if (const char *p = std::getenv("GBS_TUNING")) {
     if (*p) load_locked(p);  // a bad file leaves the table as it was
   }
-}
-
-void record_locked(const Entry &e) {
-  auto it = std::find_if(g_table.begin(), g_table.end(), [&](const Entry &x) {
-    return x.sid == e.sid && x.dtype == e.dtype && x.fma == e.fma && x.cls == e.cls;
-  });
-  if (it != g_table.end()) *it = e;
-  else g_table.push_back(e);
 }
 
 double hbm_bytes_per_s() {
@@ -169,6 +181,20 @@ bool tuned_lookup(const gbs_desc *d, int *bt, int *sl, int *bs1) {
   return true;
 }
 
+int tuned_last(const gbs_desc *d) {
+  std::lock_guard<std::mutex> lk(g_mu);
+  env_load_locked();
+  const int fma = d->fp_mode == GBS_FP_FMA ? 1 : 0;
+  const int cls = size_class(d);
+  const int mx = max_bt(d->stencil, d->dtype, fma);
+  const Entry *best = nullptr;
+  for (const Entry &e : g_last) {
+    if (e.sid != d->stencil || e.dtype != d->dtype || e.fma != fma || e.bt > mx || e.bt < 1) continue;
+    if (!best || std::abs(e.cls - cls) < std::abs(best->cls - cls)) best = &e;
+  }
+  return best && std::abs(best->cls - cls) <= 3 ? best->bt : 0;
+}
+
 }  // namespace gbs
 
 using namespace gbs;
@@ -188,13 +214,24 @@ gbs_status gbs_tune_save(const char *path) {
   FILE *f = std::fopen(path, "w");
   if (!f) return fail(GBS_ERR_INVALID, "cannot write %s", path);
   std::fprintf(f, "# stencil dtype mode size_class bt sl bs1 ms_per_step\n");
-  std::vector<Entry> t = g_table;
-  std::sort(t.begin(), t.end(), [](const Entry &a, const Entry &b) {
+  std::vector<Entry> t = g_table, last;
+  for (const Entry &e : g_last) {  // those that differ from what the other lines give
+    const bool same = std::any_of(g_table.begin(), g_table.end(), [&](const Entry &x) {
+      return x.sid == e.sid && x.dtype == e.dtype && x.fma == e.fma && x.cls == e.cls && x.bt == e.bt;
+    });
+    if (!same) last.push_back(e);
+  }
+  auto order = [](const Entry &a, const Entry &b) {
     return std::make_tuple(a.sid, a.dtype, a.fma, a.cls) < std::make_tuple(b.sid, b.dtype, b.fma, b.cls);
-  });
+  };
+  std::sort(t.begin(), t.end(), order);
+  std::sort(last.begin(), last.end(), order);
   for (const Entry &e : t)
     std::fprintf(f, "%s %s %s %d %d %d %d %.6g\n", gbs_stencil_name(e.sid), e.dtype == GBS_F64 ? "f64" : "f32",
                  e.fma ? "fma" : "exact", e.cls, e.bt, e.sl, e.bs1, e.ms);
+  for (const Entry &e : last)
+    std::fprintf(f, "%s %s %s %d %d 0 0\n", gbs_stencil_name(e.sid), e.dtype == GBS_F64 ? "f64" : "f32",
+                 e.fma ? "fma_last" : "exact_last", e.cls, e.bt);
   std::fclose(f);
   return GBS_OK;
 }
@@ -202,6 +239,7 @@ gbs_status gbs_tune_save(const char *path) {
 void gbs_tune_clear(void) {
   std::lock_guard<std::mutex> lk(g_mu);
   g_table.clear();
+  g_last.clear();
   g_env_loaded = true;
 }
 

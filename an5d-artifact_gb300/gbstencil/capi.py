@@ -133,10 +133,12 @@ def lib():
             fn = getattr(L, name)
             fn.restype = res
             fn.argtypes = args
-        # the tuning table measured on GB300 that ships with the package
-        table = Path(__file__).resolve().parent / "tuning_gb300.txt"
-        if table.exists():
-            check_with(L, L.gbs_tune_load(str(table).encode()))
+        # the tuning table measured on GB300 that ships with the package, and
+        # the degrees that fix an odd loop's last launch
+        for table in ("tuning_gb300.txt", "last_launch_gb300.txt"):
+            table = Path(__file__).resolve().parent / table
+            if table.exists():
+                check_with(L, L.gbs_tune_load(str(table).encode()))
         _lib = L
     return _lib
 

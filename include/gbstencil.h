@@ -145,7 +145,11 @@ gbs_status gbs_plan(const gbs_desc *d, gbs_plan_info *out);
  * The table is also loaded from the file named by the environment variable
  * GBS_TUNING at first use. Text format, one entry per line:
  * "<stencil> <f32|f64> <exact|fma> <size class> <bt> <sl> [<bs1>] <ms per step>"
- * (bs1: 3-D tile rows; absent or 0: the default shape). */
+ * (bs1: 3-D tile rows; absent or 0: the default shape). A line of mode
+ * fma_last or exact_last carries only the degree (0: none) that fixes the
+ * steps of a loop's last launch when its T is odd and bt is 0: after such a
+ * loop plane 0 holds the state before that launch, and a program that runs it
+ * again from there sees the same states whatever degree the table chooses. */
 typedef struct gbs_tune_candidate {
   int bt, sl;               /* sl 0: the engine's one-wave stream length */
   double redundancy;        /* computed / useful cells per launch */
@@ -206,9 +210,10 @@ typedef struct gbs_batch_stats {
  *   consecutive items in time-block order from an atomic counter, and an
  *   item waits (bounded) until its stream block and the two beside it have
  *   finished the grid's earlier time blocks (per-block completion counters).
- * GBS_BATCH_LAYERED: the same 2-D work items, one kernel node per time block
- *   in the graph, each over every grid's items of that block; kernel
- *   boundaries order the blocks, so nothing waits on the device.
+ * GBS_BATCH_LAYERED: 2-D float grids; per stencil a chain of kernel nodes in
+ *   the graph, one per time block and degree over the items of the stencil's
+ *   grids; kernel boundaries order the blocks, so nothing waits on the device,
+ *   and the chains of different stencils run side by side.
  * GBS_BATCH_STREAMS: each grid's own time loop (the single-grid kernels at
  *   the tuned degree, one kernel node per fused launch) as a chain in the
  *   graph; the chains are spread over 16 branches (environment
