@@ -71,15 +71,6 @@ __device__ __forceinline__ bool row_interior(const AdjGeom &g, int i, int j) {
   return i >= R && i < g.d0 - R && (g.dim == 2 || (j >= R && j < g.d1 - R));
 }
 
-// value of plane p at (i, j, c) (c the innermost index; 2-D: (i, c)); 0 off the grid
-template <typename T>
-__device__ __forceinline__ T ldz(const T *p, const AdjGeom &g, int i, int j, int c) {
-  if (i < 0 || i >= g.d0 || c < 0 || c >= g.last) return T(0);
-  if (g.dim == 2) return p[(long long)i * g.pitch + g.shift + c];
-  if (j < 0 || j >= g.d1) return T(0);
-  return p[((long long)i * g.d1 + j) * g.pitch + g.shift + c];
-}
-
 template <typename T, int NT> struct LinCoef {
   T c[NT];  // c_k / d
 };
@@ -150,30 +141,41 @@ __device__ __forceinline__ bool halo_cell(const AdjGeom &g, const HaloPlan &hp, 
   return true;
 }
 
-// hg(h) += sum_k c_k/d lam(h - o_k) at halo cell h
-template <class ST, typename T>
-__device__ __forceinline__ void halo_update(const AdjGeom &g, const T *lam, T *hg, const LinCoef<T, ST::kTerms> &cf,
-                                            int i, int j, int c) {
-  T acc = T(0);
-  static_for<ST::kTerms>([&](auto TI) {
-    constexpr int t = decltype(TI)::value;
-    constexpr int di = ST::kOff[t][0], dj = ST::kOff[t][1], dk = ST::kOff[t][2];
-    // 2-D offsets are (row, column); 3-D (plane, row, column)
-    const T l = ST::kDim == 2 ? ldz(lam, g, i - di, 0, c - dj) : ldz(lam, g, i - di, j - dj, c - dk);
-    acc = fma(cf.c[t], l, acc);
-  });
-  const long long o = (ST::kDim == 2 ? (long long)i * g.pitch : ((long long)i * g.d1 + j) * g.pitch) + g.shift + c;
-  hg[o] += acc;
-}
-
-// hg(h) += sum_k c_k/d lam(h - o_k) for every halo cell h
+// hg(h) += sum_k c_k/d lam(h - o_k) for every halo cell h of a 3-D grid (2-D
+// stencils of many terms too). lam is zero off the interior, so only the
+// offsets that lead there are read: which planes, rows and columns around the
+// cell are interior is found once, not per term. A face cell of a radius-1 box
+// reads 9 of its 27 neighbours; with every term bounds-checked and read, the
+// pass took longer than the step itself (j3d27pt f32, four instances of
+// 96..192 cells a side at once: 22 us a pass, 9.8 now).
 template <class ST, typename T>
 __global__ void __launch_bounds__(kAdjThreads) halo_kernel(const __grid_constant__ AdjGeom g, const T *lam, T *hg,
                                                            const __grid_constant__ LinCoef<T, ST::kTerms> cf) {
+  constexpr int R = ST::kRad, W = 2 * R + 1;
+  wait_for_previous();
   const HaloPlan hp = halo_plan(g);
   int i, j, c;
-  if (halo_cell(g, hp, (long long)blockIdx.x * kAdjThreads + threadIdx.x, i, j, c))
-    halo_update<ST, T>(g, lam, hg, cf, i, j, c);
+  if (!halo_cell(g, hp, (long long)blockIdx.x * kAdjThreads + threadIdx.x, i, j, c)) return;
+  // 2-D offsets are (row, column); 3-D (plane, row, column)
+  bool pi[W], pj[W], pc[W];
+  static_for<W>([&](auto XI) GBS_INL {
+    constexpr int x = decltype(XI)::value - R;
+    pi[x + R] = i + x >= R && i + x < g.d0 - R;
+    pj[x + R] = ST::kDim == 2 || (j + x >= R && j + x < g.d1 - R);
+    pc[x + R] = c + x >= R && c + x < g.last - R;
+  });
+  const long long line = ST::kDim == 2 ? g.pitch : (long long)g.d1 * g.pitch;  // elements per step of i
+  const long long o = (ST::kDim == 2 ? (long long)i * g.pitch : ((long long)i * g.d1 + j) * g.pitch) + g.shift + c;
+  T acc = T(0);
+  static_for<ST::kTerms>([&](auto TI) GBS_INL {
+    constexpr int t = decltype(TI)::value;
+    constexpr int di = ST::kOff[t][0], dj = ST::kDim == 2 ? 0 : ST::kOff[t][1];
+    constexpr int dk = ST::kDim == 2 ? ST::kOff[t][1] : ST::kOff[t][2];
+    const bool in = pi[R - di] && pj[R - dj] && pc[R - dk];
+    const T l = in ? lam[o - di * line - dj * g.pitch - dk] : T(0);
+    acc = fma(cf.c[t], l, acc);
+  });
+  hg[o] += acc;
 }
 
 // part[blockIdx.x][k] += sum over interior x of lam(x) u(x + o_k) / d.
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(kAdjThreads) coef_kernel(const __grid_constant
                                                            double *part, T inv_div) {
   constexpr int NT = ST::kTerms;
   constexpr int SEG = 128;
+  wait_for_previous();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int R = g.rad;
   const int width = g.last - 2 * R;
@@ -570,8 +573,8 @@ bool transposed_coefficients(const gbs_stencil_def_t *s, const std::vector<doubl
 
 // kernels of one stencil and dtype
 struct AdjKernels {
-  cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t);
-  cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t);
+  cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t, bool);
+  cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t, bool);
   cudaError_t (*grad)(const AdjGeom &, const void *, const void *, void *, void *, double *, double, double, bool,
                       cudaStream_t, bool);
 };
@@ -599,28 +602,28 @@ cudaError_t copy_halo(int dtype, const AdjGeom &g, const void *src, void *dst, i
 
 template <class ST, typename T>
 cudaError_t run_halo(const AdjGeom &g, const void *lam, void *hg, const std::vector<double> &coef, double div,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool pdl) {
   if constexpr (ST::kKind == KIND_GRADIENT) {
     return cudaErrorInvalidValue;
   } else {
     LinCoef<T, ST::kTerms> cf;
     const double dv = ST::kHasDiv ? div : 1.0;
     for (int t = 0; t < ST::kTerms; ++t) cf.c[t] = (T)(coef[t] / dv);
-    halo_kernel<ST, T><<<halo_grid(g), kAdjThreads, 0, s>>>(g, static_cast<const T *>(lam), static_cast<T *>(hg), cf);
-    return cudaGetLastError();
+    return launch_kernel(halo_kernel<ST, T>, halo_grid(g), kAdjThreads, 0, s, pdl, g, static_cast<const T *>(lam),
+                         static_cast<T *>(hg), cf);
   }
 }
 
 template <class ST, typename T>
-cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *part, double div, cudaStream_t s) {
+cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *part, double div, cudaStream_t s,
+                     bool pdl) {
   if constexpr (ST::kKind == KIND_GRADIENT || ST::kTerms > kMaxCoefGrad) {
     return cudaErrorInvalidValue;
   } else {
     const double dv = ST::kHasDiv ? div : 1.0;
     const int wave = std::min(kAdjPartRows, adj_wave(reinterpret_cast<const void *>(coef_kernel<ST, T>), kAdjThreads, 0));
-    coef_kernel<ST, T><<<wave, kAdjThreads, 0, s>>>(g, static_cast<const T *>(lam), static_cast<const T *>(u), part,
-                                                    (T)(1.0 / dv));
-    return cudaGetLastError();
+    return launch_kernel(coef_kernel<ST, T>, (unsigned)wave, kAdjThreads, 0, s, pdl, g, static_cast<const T *>(lam),
+                         static_cast<const T *>(u), part, (T)(1.0 / dv));
   }
 }
 
@@ -987,6 +990,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     cur ^= 1;
     return GBS_OK;
   };
+  BlockPlan planT{};  // the transposed step of the stencils that the forward kernels serve
   // one adjoint step lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_t) on state u_t
   auto step = [&](const char *u, bool follows) -> gbs_status {
     if (blocked) return steps(u, 1, follows);
@@ -994,9 +998,12 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s, follows),
          "adjoint: gradient2d step");
     } else {
-      CK(K.halo(g, lam[cur], hg, coef, div, s), "adjoint: halo");
-      if (dev_coef_grad) CK(K.coef(g, lam[cur], u, part, div, s), "adjoint: coefficients");
-      gbs_status r = launch_block(&dT, L, coefT.data(), div, eps, 0, 1, lam[cur], lam[cur ^ 1], s, err);
+      // each of these waits for the one before it and is launched while that ends
+      CK(K.halo(g, lam[cur], hg, coef, div, s, follows), "adjoint: halo");
+      if (dev_coef_grad) CK(K.coef(g, lam[cur], u, part, div, s, true), "adjoint: coefficients");
+      gbs_status r = GBS_OK;
+      if (planT.dim == 0) r = plan_block(&dT, L, coefT.data(), div, eps, 0, 1, false, err, &planT);
+      if (r == GBS_OK) r = launch_plan(planT, lam[cur], lam[cur ^ 1], nullptr, s, true);
       if (r != GBS_OK) return r;
     }
     cur ^= 1;
@@ -1007,7 +1014,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     // no forward state enters: T transposed steps from lam_T
     for (int left = d->timestep; left > 0;) {
       const int b = blocked ? degree(left) : 1;
-      st = blocked ? steps(nullptr, b, left < d->timestep) : step(nullptr, false);
+      st = blocked ? steps(nullptr, b, left < d->timestep) : step(nullptr, left < d->timestep);
       if (st != GBS_OK) return st;
       left -= b;
     }
@@ -1115,6 +1122,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       }
       bre = std::max(1, std::min(pi.bt, kMaxStashB));
     }
+    BlockPlan planR[kMaxStashB + 1] = {};  // the recompute's launches, by degree
     // recompute u_{t0} .. u_{t0+c-1} of chunk j into buffer j % 2 on s2
     auto recompute = [&](int j) -> gbs_status {
       const int b = j & 1;
@@ -1127,9 +1135,12 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       for (int k = 1; k < c;) {
         // one launch of bb steps from slot k-1: slots k .. k+bb-1
         const int bb = std::min(bre, c - k);
-        gbs_status r = launch_block_stash(d, L, coef.data(), div, eps, 0, bb, buf + (size_t)(k - 1) * w.plane_bytes,
-                                          buf + (size_t)(k - 1 + bb) * w.plane_bytes,
-                                          bb > 1 ? buf + (size_t)k * w.plane_bytes : nullptr, s2, err);
+        BlockPlan &plan = planR[bb];
+        gbs_status r = GBS_OK;
+        if (plan.dim == 0) r = plan_block(d, L, coef.data(), div, eps, 0, bb, bb > 1, err, &plan);
+        if (r == GBS_OK)
+          r = launch_plan(plan, buf + (size_t)(k - 1) * w.plane_bytes, buf + (size_t)(k - 1 + bb) * w.plane_bytes,
+                          bb > 1 ? buf + (size_t)k * w.plane_bytes : nullptr, s2, k > 1);
         if (r != GBS_OK) return r;
         k += bb;
       }
@@ -1147,7 +1158,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       for (int k = c - 1; k >= 0 && st == GBS_OK;) {
         const int bb = blocked ? degree(k + 1) : 1;
         const char *u = buf + (size_t)k * w.plane_bytes;
-        st = blocked ? steps(u, bb, k < c - 1) : step(u, gradient && k < c - 1);
+        st = blocked ? steps(u, bb, k < c - 1) : step(u, k < c - 1);
         k -= bb;
       }
       cudaEventRecord(freed[b], s);
