@@ -207,6 +207,20 @@ __device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&up)[PP:
   T y[V];
   bool halo_row = false;
   if constexpr (CARE == kAll) halo_row = (q < R) || (q >= p.d0 - R);
+  // the constant divisor (FMA mode folds it into the coefficients). Columns
+  // that keep their halo value are off the grid too, where memory or the ring
+  // holds anything: a 1 there, or one zero or denormal sends its warp through
+  // the rare path of the division in every row (j2d9pt-gol f32 1500^2, degree
+  // 4: 9.9 us a step, 5.8 now)
+  auto divide = [&]() GBS_INL {
+    if constexpr (ST::kHasDiv && !FMA) {
+      if constexpr (CARE != kInterior) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) y[e] = halo_row || fixed[e] ? T(1) : y[e];
+      }
+      apply_div(y, p);
+    }
+  };
   if constexpr (!ST::kAssoc) {
 #pragma unroll
     for (int e = 0; e < V; ++e) win[slot2d<PP>(PH, 2 * R)][e] = x[e];
@@ -233,7 +247,8 @@ __device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&up)[PP:
       for (int e = 0; e < V; ++e) {
         const T d = A::sub(c[e], below[e]);
         const T sd = A::mul(d, d);
-        const T s = A::add(A::add(A::add(A::add(p.eps, up[e]), sd), sr[e]), e > 0 ? sr[e > 0 ? e - 1 : 0] : sl);
+        T s = A::add(A::add(A::add(A::add(p.eps, up[e]), sd), sr[e]), e > 0 ? sr[e > 0 ? e - 1 : 0] : sl);
+        if constexpr (CARE != kInterior) s = halo_row || fixed[e] ? T(1) : s;  // as for the quotients below
         up[e] = sd;
         y[e] = gradient_finish<T, FMA>(c[e], s, p.coef[0]);
       }
@@ -256,7 +271,7 @@ __device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&up)[PP:
           else y[e] = term_next<T, FMA>(y[e], p.coef[t], a);
         });
       });
-      if constexpr (ST::kHasDiv && !FMA) apply_div(y, p);  // FMA mode: folded into the coefficients
+      divide();
     }
     if constexpr (CARE != kInterior) {
 #pragma unroll
@@ -296,7 +311,7 @@ __device__ __forceinline__ void level2d(T (&win)[PP::WSLOTS][PP::V], T (&up)[PP:
     constexpr int oslot = slot2d<PP>(PH, 0);
 #pragma unroll
     for (int e = 0; e < V; ++e) y[e] = win[oslot][e];
-    if constexpr (ST::kHasDiv && !FMA) apply_div(y, p);  // FMA mode: folded into the coefficients
+    divide();
     if constexpr (CARE != kInterior) {
 #pragma unroll
       for (int e = 0; e < V; ++e) y[e] = (halo_row || fixed[e]) ? cv[e] : y[e];

@@ -16,6 +16,18 @@ from . import capi
 TORCH_DT = {np.dtype(np.float32): torch.float32, np.dtype(np.float64): torch.float64}
 
 
+# the current stream's handle without a Stream object around it (9 us of a
+# small run's 23); the public way where torch has no such call
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def current_stream(device) -> int:
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
+
+
 class DeviceGrid:
     def __init__(self, name: str, dtype, n, device=None):
         self.name = name
@@ -29,6 +41,10 @@ class DeviceGrid:
         self.device = torch.device(device or "cuda")
         self.buf = torch.zeros(self.layout.bytes // es, dtype=TORCH_DT[self.dtype], device=self.device)
         assert self.buf.data_ptr() % 128 == 0
+        # shape, strides and offset of a plane's view
+        L = self.layout
+        row = (L.pitch,) if self.dim == 2 else (L.dimsize[1] * L.pitch, L.pitch)
+        self._view = (tuple(self.dimsize), row + (1,), L.shift, L.plane)
 
     @property
     def dimsize(self):
@@ -36,13 +52,10 @@ class DeviceGrid:
 
     def plane(self, p: int) -> torch.Tensor:
         """Strided view of time plane p with shape dimsize."""
-        L = self.layout
-        flat = self.buf[p * L.plane:(p + 1) * L.plane]
-        if self.dim == 2:
-            v = flat.view(L.dimsize[0], L.pitch)
-        else:
-            v = flat.view(L.dimsize[0], L.dimsize[1], L.pitch)
-        return v[..., L.shift:L.shift + L.dimsize[self.dim - 1]]
+        if p not in (0, 1):
+            raise IndexError("a grid has planes 0 and 1")
+        size, stride, shift, plane = self._view
+        return self.buf.as_strided(size, stride, self.buf.storage_offset() + p * plane + shift)
 
     def desc(self, timestep, fp_mode="fma", bt=0, sl=0, coef=None, divisor=0.0, eps=0.0, bs1=0):
         return capi.make_desc(self.name, self.dtype, self.n, timestep, fp_mode, bt, sl, bs1=bs1,
@@ -76,6 +89,6 @@ class DeviceGrid:
             stream: int | None = None, bs1=0):
         """Enqueues the time loop on ``stream`` (default: torch's current)."""
         d, keep = self.desc(timestep, fp_mode, bt, sl, coef, divisor, eps, bs1)
-        s = torch.cuda.current_stream(self.device).cuda_stream if stream is None else stream
+        s = current_stream(self.buf.device) if stream is None else stream
         capi.run_device(d, self.buf.data_ptr(), s)
         return keep

@@ -70,10 +70,11 @@ def entries() -> int:
 
 
 # Sizes the shipped table covers: every stencil at the artifact's benchmark
-# sizes (compiled/run.sh: 2-D 16384^2, 3-D 512^3) and at the sizes of the
-# single-grid workloads (2-D 4096^2 and 2048^2, 3-D 384^3 and 256^3), and
-# small grids, whose launches are bound by latency.
-TABLE_SIZES = {2: [4096, 16384, 2048, 1024, 256], 3: [512, 384, 256, 128, 64]}
+# sizes (compiled/run.sh: 2-D 16384^2, 3-D 512^3), at the sizes of the
+# single-grid workloads (2-D 4096^2 and 2048^2, 3-D 384^3 and 256^3), at one
+# size of every 2-D size class from 2^16 to 2^24 cells, where the best degree
+# moves fastest, and at small 3-D grids, whose launches are bound by latency.
+TABLE_SIZES = {2: [4096, 16384, 2048, 1024, 256, 431, 609, 861, 1722, 3444, 8192], 3: [512, 384, 256, 128, 64]}
 
 
 def main():
