@@ -70,15 +70,8 @@ __device__ __forceinline__ void apply_div(T (&y)[V], const Params2D<T, NT> &p) {
     }
   }
   if (p.divmode == 0) return;
-#pragma unroll 1
-  for (int e = 0; e < V; ++e) {  // one copy of the long checked division
-    T v = y[0];
 #pragma unroll
-    for (int k = 1; k < V; ++k) v = k == e ? y[k] : v;
-    v = div_by(v, p.div, p.rdiv);
-#pragma unroll
-    for (int k = 0; k < V; ++k) y[k] = k == e ? v : y[k];
-  }
+  for (int e = 0; e < V; ++e) y[e] = div_by(y[e], p.div, p.rdiv);
 }
 
 // Compile-time facts about a stencil's term list.
