@@ -87,6 +87,12 @@ template <class ST, int B, bool COEF> struct AdjPipe2D {
                           SMEM = RINGS > SUMS ? RINGS : SUMS;
   static constexpr int ML = (B * R + V - 1) / V * V;
   static constexpr int WOUT = (COLS - ML - B * R) / V * V;
+  // Single steps in double: the FP64 pipe bounds them, so the rows before a
+  // block's first are not computed: whole groups that only fill the window come
+  // first, and the rows after them need no branch (a branch per row instead kept
+  // the compiler from overlapping rows: box2d2r 1500^2 6494 us against 5266)
+  static constexpr bool FILL = B == 1 && sizeof(T) == 8;
+  static constexpr int NFILL = FILL ? (2 * R + NPH - 1) / NPH : 0;
   static constexpr int slot(int ph, int j) { return ROT ? (ph + 1 + j) % W : ph + j; }
 };
 
@@ -115,8 +121,11 @@ __device__ __forceinline__ void extend(T (&ext)[V + 2 * R], const T (&row)[V], i
   });
 }
 
+// In double two CTAs on an SM fill the FP64 pipe; asking for no more keeps the
+// box of radius 2 from spilling its coefficient sums (560 bytes of 168 registers)
 template <class ST, int B, bool COEF>
-__global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constant__ AdjParams2D<ST::kTerms> p) {
+__global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2 : 0))
+    adj2d_kernel(const __grid_constant__ AdjParams2D<ST::kTerms> p) {
   using AP = AdjPipe2D<ST, B, COEF>;
   constexpr int V = AP::V, R = AP::R, NPH = AP::NPH, PG = AP::PG, NT = ST::kTerms;
   constexpr int NP = COEF ? NT : 1, NL = COEF ? B : 1;
@@ -159,10 +168,10 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
     }
     const int i0 = R + blk * sl, i1 = min(i0 + sl, p.d0 - R);
     const int o0 = blk == 0 ? 0 : i0, o1 = blk == nblocks - 1 ? p.d0 : i1;  // rows owned
-    const int pstart = max(0, o0 - B * R), pend = min(p.d0, o1 + B * R);
+    const int pstart = AP::FILL ? o0 + R - AP::NFILL * NPH : max(0, o0 - B * R), pend = min(p.d0, o1 + B * R);
     const int ng = (o1 + B * R - pstart + NPH - 1) / NPH;
     // rows [fast_lo, fast_hi): every row that enters or leaves a level is interior
-    const int fast_lo = o0 - B * R >= R ? pstart : (B + 1) * R;
+    const int fast_lo = pstart >= R ? pstart : (B + 1) * R;
     const int fast_hi = o1 + B * R <= p.d0 - R ? 0x7fffffff : p.d0 - R;
     const unsigned nown = (unsigned)(o1 - o0), nout = (unsigned)(i1 - i0);
 
@@ -180,7 +189,7 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
     auto request_group = [&]() GBS_INL {
 #pragma unroll
       for (int ph = 0; ph < NPH; ++ph) {
-        if (in_row && req + ph < pend) cp_async16(my_s + wr + ph * AP::ROWB, lam_next);
+        if (in_row && (AP::FILL ? (unsigned)(req + ph) < (unsigned)pend : req + ph < pend)) cp_async16(my_s + wr + ph * AP::ROWB, lam_next);
         lam_next += p.pitch;
         if constexpr (COEF) {
 #pragma unroll
@@ -209,8 +218,9 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
     int pb = pstart;
     T *out = p.lam_out + ((long long)(pstart - B * R) * p.pitch + el);  // the row the last level completes
 
-    auto rows = [&](auto CAREI) GBS_INL {
+    auto rows = [&](auto CAREI, auto FILLI) GBS_INL {
       constexpr int care = decltype(CAREI)::value;
+      constexpr bool fill = decltype(FILLI)::value;
       static_for<NPH>([&](auto PHI) GBS_INL {
         constexpr int ph = decltype(PHI)::value;
         const int pp = pb + ph;
@@ -235,8 +245,9 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
             T row[V];
 #pragma unroll
             for (int e = 0; e < V; ++e) row[e] = win[l][AP::slot(ph, R)][e];
-            extend<V, R, care != kIn>(ext, row, lane);
+            if constexpr (!fill) extend<V, R, care != kIn>(ext, row, lane);
           }
+          if constexpr (fill) return;
           // lam^l(y - o_t) for the lane's element e of row q
           auto operand = [&](auto TI, auto EI) GBS_INL -> T {
             constexpr int di = ST::kOff[decltype(TI)::value][0], dj = ST::kOff[decltype(TI)::value][1];
@@ -288,9 +299,9 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
 #pragma unroll
           for (int e = 0; e < V; ++e) x[e] = y[e];
         });
-        const bool keep = (unsigned)(pp - B * R - i0) < nout;
-        st_vec_global_if<V>(out, x, keep && whole);
-        if constexpr (care != kIn) {
+        [[maybe_unused]] const bool keep = (unsigned)(pp - B * R - i0) < nout;
+        if constexpr (!fill) st_vec_global_if<V>(out, x, keep && whole);
+        if constexpr (care != kIn && !fill) {
 #pragma unroll
           for (int e = 0; e < V; ++e) st_global_if(out + e, x[e], keep && !whole && col0 + e >= cs && col0 + e < ce);
         }
@@ -310,9 +321,10 @@ __global__ void __launch_bounds__(kWarps * 32) adj2d_kernel(const __grid_constan
     for (int k = 0; k < ng; ++k) {
       request_group();
       cp_async_wait<PG>();
-      if (pb < fast_lo || pb + NPH > fast_hi) rows(IC<kEverything>());
-      else if (edge) rows(IC<kCols>());
-      else rows(IC<kIn>());
+      if (k < AP::NFILL) rows(IC<kEverything>(), IC<1>());
+      else if (pb < fast_lo || pb + NPH > fast_hi) rows(IC<kEverything>(), IC<0>());
+      else if (edge) rows(IC<kCols>(), IC<0>());
+      else rows(IC<kIn>(), IC<0>());
       pb += NPH;
       rd = rd + AP::GROUP == AP::RING ? 0u : rd + AP::GROUP;
     }
@@ -378,6 +390,28 @@ template <class ST, bool COEF> constexpr int max_degree() {
   return 1;
 }
 
+// Rows per block of a step in double: whole groups (a rest would be computed
+// all the same), the FP64 pipe shared by the warps of an SM quarter. extra: what a
+// block costs beside its rows, in rows.
+inline int fill_rows(int nstrips, int ni, int group, int extra) {
+  const int sms = sm_count();
+  double best = 1e300;
+  int best_sl = ni;
+  for (int k = 1; k <= 32; ++k) {
+    const long long nb = std::max<long long>(1, std::min<long long>(ni, (long long)k * sms * kWarps / nstrips));
+    const int sl = (int)((ni + nb - 1) / nb + group - 1) / group * group;
+    const long long ctas = (((long long)ni + sl - 1) / sl * nstrips + kWarps - 1) / kWarps;
+    const double per_sm = (double)((ctas + sms - 1) / sms);
+    const double cost = (sl + extra) * std::max(1.3, per_sm);  // a warp alone does not fill the pipe
+    if (cost < best) {
+      best = cost;
+      best_sl = sl;
+    }
+    if (nb == ni) break;
+  }
+  return best_sl;
+}
+
 template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cudaStream_t stream) {
   using AP = AdjPipe2D<ST, B, COEF>;
   auto kern = adj2d_kernel<ST, B, COEF>;
@@ -411,18 +445,20 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   const int wave = adj_wave(reinterpret_cast<const void *>(adj2d_kernel<ST, M, COEF>), kWarps * 32,
                             AdjPipe2D<ST, M, COEF>::SMEM);
   // a block's sums cost about as much as a dozen rows (radius 1)
-  int sl = stream_rows_2d(p.nstrips, ni, M * ST::kRad + (COEF ? 6 : 0), sizeof(T) == 8, (long long)wave * kWarps);
+  int sl = AP::FILL ? fill_rows(p.nstrips, ni, AP::NPH, COEF ? 9 : 3)
+                    : stream_rows_2d(p.nstrips, ni, M * ST::kRad + (COEF ? 6 : 0), false, (long long)wave * kWarps);
   // The edge strips' rows cost more (masks, halo gradient), and all warps start
   // together: without products, a third of the rows per block there (four
   // steps of a 2048^2 grid 21.8 us with the same rows, 18.6 with half, 14.8
   // with a third); with products, which every row has, the same (two steps
-  // 19.3, 20.1, 21.0 us).
+  // 19.3, 20.1, 21.0 us). In double, bound by the FP64 pipe, the same as well
+  // (star2d1r 1500^2, 20 steps with the forward pass: 1512 us with a third, 1301).
   const int edges = p.nstrips > 1 ? 2 : 1;
   long long grid = 0;
-  for (;; ++sl) {  // one row of the partial-sum table per CTA
+  for (;; sl += AP::FILL ? AP::NPH : 1) {  // one row of the partial-sum table per CTA
     p.sl = sl;
     p.nblocks = (ni + sl - 1) / sl;
-    p.sl_e = COEF ? sl : (sl + 2) / 3;
+    p.sl_e = COEF || AP::FILL ? sl : (sl + 2) / 3;
     p.nblocks_e = (ni + p.sl_e - 1) / p.sl_e;
     grid = ((long long)edges * p.nblocks_e + (long long)(p.nstrips - edges) * p.nblocks + kWarps - 1) / kWarps;
     if (grid <= kAdjPartRows || sl >= ni) break;

@@ -237,7 +237,7 @@ std::vector<int> loop_steps(const gbs_desc *d, int bt) {
   return out;
 }
 
-static int sm_count() {
+int sm_count() {
   static int n = -1;
   if (n < 0) {
     int dev = 0, v = 0;

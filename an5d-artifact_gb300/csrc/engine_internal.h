@@ -57,6 +57,7 @@ std::vector<int> loop_steps(const gbs_desc *d, int bt);
 // resident_warps: warps the GPU holds at once for this kernel (0 = unknown)
 // rows per stream block of a 2-D launch of nstrips strips over ni rows whose
 // blocks overlap by br rows at each end
+int sm_count();
 int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps);
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident_warps);
 long long resident_warps_2d(int sid, int dtype, int fma, int b);
