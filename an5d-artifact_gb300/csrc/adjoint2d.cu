@@ -248,6 +248,9 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
             if constexpr (!fill) extend<V, R, care != kIn>(ext, row, lane);
           }
           if constexpr (fill) return;
+          if constexpr (AP::FILL && care == kEverything) {  // rows past the block's last
+            if ((unsigned)(q - o0) >= nown) return;
+          }
           // lam^l(y - o_t) for the lane's element e of row q
           auto operand = [&](auto TI, auto EI) GBS_INL -> T {
             constexpr int di = ST::kOff[decltype(TI)::value][0], dj = ST::kOff[decltype(TI)::value][1];
@@ -322,7 +325,7 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
       request_group();
       cp_async_wait<PG>();
       if (k < AP::NFILL) rows(IC<kEverything>(), IC<1>());
-      else if (pb < fast_lo || pb + NPH > fast_hi) rows(IC<kEverything>(), IC<0>());
+      else if (pb < fast_lo || pb + NPH > fast_hi || (AP::FILL && pb + NPH > o1 + R)) rows(IC<kEverything>(), IC<0>());
       else if (edge) rows(IC<kCols>(), IC<0>());
       else rows(IC<kIn>(), IC<0>());
       pb += NPH;
@@ -390,16 +393,15 @@ template <class ST, bool COEF> constexpr int max_degree() {
   return 1;
 }
 
-// Rows per block of a step in double: whole groups (a rest would be computed
-// all the same), the FP64 pipe shared by the warps of an SM quarter. extra: what a
-// block costs beside its rows, in rows.
-inline int fill_rows(int nstrips, int ni, int group, int extra) {
+// Rows per block of a step in double: the FP64 pipe is shared by the warps of an
+// SM quarter. extra: what a block costs beside its rows, in rows.
+inline int fill_rows(int nstrips, int ni, int extra) {
   const int sms = sm_count();
   double best = 1e300;
   int best_sl = ni;
   for (int k = 1; k <= 32; ++k) {
     const long long nb = std::max<long long>(1, std::min<long long>(ni, (long long)k * sms * kWarps / nstrips));
-    const int sl = (int)((ni + nb - 1) / nb + group - 1) / group * group;
+    const int sl = (int)((ni + nb - 1) / nb);
     const long long ctas = (((long long)ni + sl - 1) / sl * nstrips + kWarps - 1) / kWarps;
     const double per_sm = (double)((ctas + sms - 1) / sms);
     const double cost = (sl + extra) * std::max(1.3, per_sm);  // a warp alone does not fill the pipe
@@ -445,7 +447,7 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   const int wave = adj_wave(reinterpret_cast<const void *>(adj2d_kernel<ST, M, COEF>), kWarps * 32,
                             AdjPipe2D<ST, M, COEF>::SMEM);
   // a block's sums cost about as much as a dozen rows (radius 1)
-  int sl = AP::FILL ? fill_rows(p.nstrips, ni, AP::NPH, COEF ? 9 : 3)
+  int sl = AP::FILL ? fill_rows(p.nstrips, ni, COEF ? 9 : 3)
                     : stream_rows_2d(p.nstrips, ni, M * ST::kRad + (COEF ? 6 : 0), false, (long long)wave * kWarps);
   // The edge strips' rows cost more (masks, halo gradient), and all warps start
   // together: without products, a third of the rows per block there (four
@@ -455,7 +457,7 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   // (star2d1r 1500^2, 20 steps with the forward pass: 1512 us with a third, 1301).
   const int edges = p.nstrips > 1 ? 2 : 1;
   long long grid = 0;
-  for (;; sl += AP::FILL ? AP::NPH : 1) {  // one row of the partial-sum table per CTA
+  for (;; ++sl) {  // one row of the partial-sum table per CTA
     p.sl = sl;
     p.nblocks = (ni + sl - 1) / sl;
     p.sl_e = COEF || AP::FILL ? sl : (sl + 2) / 3;
