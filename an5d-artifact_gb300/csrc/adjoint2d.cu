@@ -60,6 +60,7 @@ template <int NT> struct AdjParams2D {
   int d0, d1, shift, nstrips;
   int nblocks, sl;           // stream blocks of the inner strips, their rows
   int nblocks_e, sl_e;       // of the edge strips
+  long long item0;           // the launch's first item
   T inv_div;
   T coef[NT];                // c_k / d
 };
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
   __shared__ double sums[NL * NP];
   wait_for_previous();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long gw = (long long)blockIdx.x * kWarps + wid;
+  const long long gw = p.item0 + (long long)blockIdx.x * kWarps + wid;
   // this CTA's row of the partial sums, read ahead of its update
   double total = 0.0;
   if (COEF && (int)threadIdx.x < NT) total = p.part[(size_t)blockIdx.x * NT + threadIdx.x];
@@ -456,16 +457,26 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   // 19.3, 20.1, 21.0 us). In double, bound by the FP64 pipe, the same as well
   // (star2d1r 1500^2, 20 steps with the forward pass: 1512 us with a third, 1301).
   const int edges = p.nstrips > 1 ? 2 : 1;
-  long long grid = 0;
-  for (;; ++sl) {  // one row of the partial-sum table per CTA
+  // With products every CTA of a launch has its own row of the partial-sum
+  // table: blocks as long as that takes, and where one block per strip is
+  // still too many (more than 4096 strips), several launches over the items.
+  constexpr long long kMost = (long long)kAdjPartRows * kWarps;
+  long long items = 0;
+  for (;; ++sl) {
     p.sl = sl;
     p.nblocks = (ni + sl - 1) / sl;
     p.sl_e = COEF || AP::FILL ? sl : (sl + 2) / 3;
     p.nblocks_e = (ni + p.sl_e - 1) / p.sl_e;
-    grid = ((long long)edges * p.nblocks_e + (long long)(p.nstrips - edges) * p.nblocks + kWarps - 1) / kWarps;
-    if (grid <= kAdjPartRows || sl >= ni) break;
+    items = (long long)edges * p.nblocks_e + (long long)(p.nstrips - edges) * p.nblocks;
+    if (items <= kMost || sl >= ni) break;
   }
-  return launch_kernel(kern, (unsigned)grid, kWarps * 32, smem, stream, a.pdl, p);
+  const long long most = COEF ? kMost : items;
+  for (p.item0 = 0; p.item0 < items; p.item0 += most) {
+    const unsigned grid = (unsigned)((std::min(most, items - p.item0) + kWarps - 1) / kWarps);
+    const cudaError_t e = launch_kernel(kern, grid, kWarps * 32, smem, stream, a.pdl || p.item0 > 0, p);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 template <class ST, bool COEF> void fill(AdjStep2DFn (&f)[kAdjMaxB + 1]) {
