@@ -271,7 +271,7 @@ constexpr int kGradWarps = 4;
 template <class ST, typename T>
 __global__ void __launch_bounds__(kGradWarps * 32)
     grad2d_kernel(const __grid_constant__ AdjGeom g, const T *u, const T *lam, T *lam_out, T *hg, double *part, T num,
-                  T eps, int want_coef, int nstrips, int nblocks, int sl) {
+                  T eps, int want_coef, int nstrips, int nblocks, int sl, long long item0) {
   using GP = GradPipe<ST, T>;
   using A = Arith<T>;
   constexpr int V = GP::V, R = 1, NPH = GP::NPH, PG = GP::PG;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kGradWarps * 32)
   __shared__ double red[kGradWarps];
   wait_for_previous();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long gw = (long long)blockIdx.x * kGradWarps + wid;
+  const long long gw = item0 + (long long)blockIdx.x * kGradWarps + wid;
   double pnum = 0.0;
   if (gw < (long long)nstrips * nblocks) {
     const int strip = (int)(gw % nstrips), blk = (int)(gw / nstrips);
@@ -638,13 +638,22 @@ cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam
     const int ni = g.d0 - 2, nstrips = (g.d1 - 2 + GP::WOUT - 1) / GP::WOUT;
     const int wave = adj_wave(reinterpret_cast<const void *>(grad2d_kernel<ST, T>), kGradWarps * 32, 0);
     int sl = stream_rows_2d(nstrips, ni, 2, sizeof(T) == 8, (long long)wave * kGradWarps);
-    // one partial-sum row per CTA
-    while (((long long)nstrips * ((ni + sl - 1) / sl) + kGradWarps - 1) / kGradWarps > kAdjPartRows) ++sl;
+    // with the sum for num every CTA has its own row of the partial-sum table:
+    // blocks as long as that takes, and where one block per strip is still too
+    // many (more than 4096 strips), several launches over the items
+    constexpr long long kMost = (long long)kAdjPartRows * kGradWarps;
+    while (sl < ni && (long long)nstrips * ((ni + sl - 1) / sl) > kMost) ++sl;
     const int nblocks = (ni + sl - 1) / sl;
-    const unsigned grid = (unsigned)(((long long)nstrips * nblocks + kGradWarps - 1) / kGradWarps);
-    return launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, pdl, g, static_cast<const T *>(u),
-                         static_cast<const T *>(lam), static_cast<T *>(lam_out), static_cast<T *>(hg), part, (T)num,
-                         (T)eps, want_coef ? 1 : 0, nstrips, nblocks, sl);
+    const long long items = (long long)nstrips * nblocks, most = want_coef ? kMost : items;
+    for (long long item0 = 0; item0 < items; item0 += most) {
+      const unsigned grid = (unsigned)((std::min(most, items - item0) + kGradWarps - 1) / kGradWarps);
+      const cudaError_t e =
+          launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, pdl || item0 > 0, g,
+                        static_cast<const T *>(u), static_cast<const T *>(lam), static_cast<T *>(lam_out),
+                        static_cast<T *>(hg), part, (T)num, (T)eps, want_coef ? 1 : 0, nstrips, nblocks, sl, item0);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }
 }
 

@@ -16,3 +16,9 @@ pytestmark = pytest.mark.gpu
 ], ids=str)
 def test_linear_wide(name, dtype, n):
     check(name, dtype, n, 3, 2, 21)
+
+
+@pytest.mark.parametrize("dtype,n", [(np.float64, (1, 245761)), (np.float64, (3, 300001)), (np.float32, (2, 491521))],
+                         ids=str)
+def test_gradient2d_wide(dtype, n):
+    check("gradient2d", dtype, n, 3, 2, 22)
