@@ -800,7 +800,10 @@ gbs_status on_branches(int n, cudaStream_t stream, F run) {
 }  // namespace
 
 // computed once per (device ordinal, kernel): a process may drive GPUs with
-// different SM counts
+// different SM counts. The kernel is opted in to its shared memory first: the
+// query holds no CTA of one that is not (above 48 KB), and the answer, which
+// decides the blocks of a step and with them the order of its sums, must not
+// depend on whether the kernel has been launched before.
 int adj_wave(const void *kernel, int threads, size_t smem) {
   static std::mutex mu;
   static std::map<std::pair<int, const void *>, int> cache;
@@ -814,6 +817,8 @@ int adj_wave(const void *kernel, int threads, size_t smem) {
   if (it != cache.end()) return it->second;
   int nb = 0, sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      (smem > kOptInSmem &&
+       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) != cudaSuccess || nb <= 0) {
     (void)cudaGetLastError();
     return kAdjPartRows;

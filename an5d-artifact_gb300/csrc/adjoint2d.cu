@@ -419,7 +419,7 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   using AP = AdjPipe2D<ST, B, COEF>;
   auto kern = adj2d_kernel<ST, B, COEF>;
   constexpr size_t smem = AP::SMEM;
-  if (smem > 40 * 1024) {  // 48 KB by default, with the kernel's static part
+  if (smem > kOptInSmem) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();

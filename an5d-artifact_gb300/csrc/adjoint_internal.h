@@ -38,7 +38,11 @@ struct AdjPicks2D {
 GBS_FOR_EACH_ADJ2D(GBS_ADJ2D_DECL)
 #undef GBS_ADJ2D_DECL
 
-// CTAs of `kernel` that the current device holds at once
+// dynamic shared memory above which the adjoint's kernels are opted in (48 KB
+// is the default, with a kernel's static part)
+constexpr size_t kOptInSmem = 40 * 1024;
+
+// CTAs of `kernel` that the current device holds at once (smem: dynamic)
 int adj_wave(const void *kernel, int threads, size_t smem);
 
 }  // namespace gbs
