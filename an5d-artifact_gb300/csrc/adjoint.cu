@@ -244,7 +244,9 @@ __global__ void __launch_bounds__(kAdjThreads) coef_kernel(const __grid_constant
 // Jacobian: -w(y) sum_n d_n(y) and the neighbours' c q^3 d_n share their
 // differences). A term belongs to the edge between two cells and enters both
 // with opposite sign, so each edge's difference, square and flux is formed
-// once. At a halo cell the same sum is the increment of its gradient.
+// once. At a halo cell the same sum is the increment of its gradient. An edge
+// without an interior end has no term: its difference is set to 0 before it
+// meets w + w = 0, for its states may be infinite or NaN.
 //
 // A warp owns a strip of output columns and a block of output rows and
 // streams the rows of u and lam like the 2-D stencil kernels: every lane
@@ -289,13 +291,13 @@ __global__ void __launch_bounds__(kGradWarps * 32)
     const int el = cs + g.shift - GP::ML + lane * V;
     const int col0 = el - g.shift;
     const bool in_row = el >= 0 && el + V <= g.pitch;
-    bool on[V], inner[V], sum_col[V];
+    bool inner[V], hedge[V], sum_col[V];  // hedge: an end of the edge to column e + 1 is an interior column
     bool whole = true;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
       const int c = col0 + e;
-      on[e] = c >= 0 && c < g.d1;
       inner[e] = c >= R && c < g.d1 - R;
+      hedge[e] = c >= R - 1 && c < g.d1 - R;
       sum_col[e] = c >= cs && c < ce;
       whole = whole && sum_col[e];
     }
@@ -341,24 +343,22 @@ __global__ void __launch_bounds__(kGradWarps * 32)
         T x[V], lx[V];
         ld_vec<T, V>(x, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB));
         ld_vec<T, V>(lx, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB + 512));
-        const bool row_on = pp < g.d0;
-        // off the grid u is 0, so that 0 * (u(x) - u(y)) is 0 there
-#pragma unroll
-        for (int e = 0; e < V; ++e) x[e] = row_on && on[e] ? x[e] : T(0);
         const bool row_in = pp - 1 >= R && pp - 1 < g.d0 - R;  // row p-1 is interior
+        const bool vedge = pp >= R && pp - 1 < g.d0 - R;       // row p-1 or row p is
         // horizontal edges of row p-1 (e: between columns e and e+1)
         T dh[V], sh[V];
         const T after = row_elem<V, V>(u1);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           dh[e] = A::sub(e + 1 < V ? u1[e + 1 < V ? e + 1 : e] : after, u1[e]);
+          dh[e] = row_in && hedge[e] ? dh[e] : T(0);
           sh[e] = A::mul(dh[e], dh[e]);
         }
         const T sleft = shfl_up(sh[V - 1], 1);
         T dn[V], sn[V], w1[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          dn[e] = A::sub(x[e], u1[e]);
+          dn[e] = vedge && inner[e] ? A::sub(x[e], u1[e]) : T(0);
           sn[e] = A::mul(dn[e], dn[e]);
           const T s = A::add(A::add(A::add(A::add(eps, sv[e]), sn[e]), sh[e]), e > 0 ? sh[e > 0 ? e - 1 : 0] : sleft);
           const T q = rsqrt_near(s);

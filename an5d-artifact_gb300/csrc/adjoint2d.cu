@@ -7,7 +7,11 @@
 //   and, for the coefficient gradients, acc_k += lam^l(y - o_k) u_{t-l}(y)
 // over every cell y: sum_x lam(x) u(x + o_k) with the states' cells as the
 // index of the sum, so that the products use the very operands of the step
-// and read one row of the state, with no neighbours.
+// and read one row of the state, with no neighbours. Where y - o_k is not
+// interior lam is 0, and so is the product, unless the state there is infinite
+// or NaN: a warp at the grid's rim whose sums are not finite forms them again
+// without those products (recount; tests of every product in the row loops
+// cost 10 to 13%, j2d5pt and j2d9pt f32 2048^2).
 //
 // A warp owns a strip of columns and a block of rows and streams the rows as
 // the forward kernels do (kernel2d.cuh): lane-private cp.async copies of lam's
@@ -109,6 +113,84 @@ template <typename U> __device__ __forceinline__ void pair_add(U &hi, U &lo, U v
   hi = s;
 }
 
+// A warp's work item: a strip of columns and a block of rows.
+struct AdjItem {
+  int cs, ce;          // columns stored
+  int own_lo, own_hi;  // and those summed over (a grid's edge strips own the halo beside them)
+  int i0, i1, o0, o1;  // the same for the rows
+  bool rim;            // owns halo cells
+};
+// the edge strips' items come first, in shorter blocks (see launch)
+template <class ST, class AP> __device__ __forceinline__ AdjItem adj_item(const AdjParams2D<ST::kTerms> &p, long long gw) {
+  constexpr int R = ST::kRad;
+  const int edges = p.nstrips > 1 ? 2 : 1;
+  const long long edge_items = (long long)edges * p.nblocks_e;
+  const bool first = gw < edge_items;
+  const int strip = first ? (gw % edges ? p.nstrips - 1 : 0) : 1 + (int)((gw - edge_items) % (p.nstrips - edges));
+  const int blk = first ? (int)(gw / edges) : (int)((gw - edge_items) / (p.nstrips - edges));
+  const int sl = first ? p.sl_e : p.sl, nblocks = first ? p.nblocks_e : p.nblocks;
+  AdjItem it;
+  it.cs = R + strip * AP::WOUT;
+  it.ce = min(it.cs + AP::WOUT, p.d1 - R);
+  it.own_lo = strip == 0 ? 0 : it.cs;
+  it.own_hi = strip == p.nstrips - 1 ? p.d1 : it.ce;
+  it.i0 = R + blk * sl;
+  it.i1 = min(it.i0 + sl, p.d0 - R);
+  it.o0 = blk == 0 ? 0 : it.i0;
+  it.o1 = blk == nblocks - 1 ? p.d0 : it.i1;
+  it.rim = first || blk == 0 || blk == nblocks - 1;
+  return it;
+}
+
+// One lane's sum (hi, lo) for term t of level l, in the order of the row loops
+// and with lam^l as the step forms it, over the cells y whose y - o_t is
+// interior. Plain loads and loops: for states that are not finite.
+template <class ST, class AP>
+__device__ __noinline__ void recount(const AdjParams2D<ST::kTerms> &p, long long gw, int l, int t, T &hi, T &lo) {
+  constexpr int R = ST::kRad, V = AP::V;
+  const AdjItem it = adj_item<ST, AP>(p, gw);
+  const int col0 = it.cs - AP::ML + (int)(threadIdx.x & 31) * V;
+  auto offset = [](int k, int &di, int &dj) GBS_INL {
+    static_for<ST::kTerms>([&](auto TI) GBS_INL {
+      constexpr int kk = decltype(TI)::value, ki = ST::kOff[kk][0], kj = ST::kOff[kk][1];
+      if (kk == k) {
+        di = ki;
+        dj = kj;
+      }
+    });
+  };
+  auto inner = [&](int i, int j) GBS_INL { return i >= R && i < p.d0 - R && j >= R && j < p.d1 - R; };
+  auto lam = [&](int i, int j) GBS_INL { return inner(i, j) ? __ldcg(p.lam + (long long)i * p.pitch + p.shift + j) : T(0); };
+  int di = 0, dj = 0;
+  offset(t, di, dj);
+  T acc = T(0);
+  hi = lo = T(0);
+#pragma unroll 1
+  for (int q = it.o0; q < it.o1; ++q) {
+#pragma unroll 1
+    for (int c = max(col0, it.own_lo); c < min(col0 + V, it.own_hi); ++c) {
+      const int i = q - di, j = c - dj;
+      if (!inner(i, j)) continue;
+      T v = lam(i, j);
+      if (l == 1) {
+#pragma unroll 1
+        for (int k = 0; k < ST::kTerms; ++k) {
+          int ki = 0, kj = 0;
+          offset(k, ki, kj);
+          const T a = lam(i - ki, j - kj);
+          v = k == 0 ? Arith<T>::mul(p.coef[0], a) : Arith<T>::fma(p.coef[k], a, v);
+        }
+      }
+      acc = Arith<T>::fma(v, __ldcg(p.u - (long long)l * p.u_stride + (long long)q * p.pitch + p.shift + c), acc);
+    }
+    if (sizeof(T) == 4 && (q - it.o0) % kFlushRows == kFlushRows - 1) {
+      pair_add(hi, lo, acc);
+      acc = T(0);
+    }
+  }
+  pair_add(hi, lo, acc);
+}
+
 // A row extended by its in-row neighbours. Beyond the window they are 0 (only
 // a halo column's own neighbours off the grid are ever that far).
 template <int V, int R, bool ZERO>
@@ -138,10 +220,9 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
   // this CTA's row of the partial sums, read ahead of its update
   double total = 0.0;
   if (COEF && (int)threadIdx.x < NT) total = p.part[(size_t)blockIdx.x * NT + threadIdx.x];
-  // the edge strips' items come first, in shorter blocks (see launch)
   const int edges = p.nstrips > 1 ? 2 : 1;
-  const long long edge_items = (long long)edges * p.nblocks_e;
-  const bool busy = gw < edge_items + (long long)(p.nstrips - edges) * p.nblocks;
+  const bool busy = gw < (long long)edges * p.nblocks_e + (long long)(p.nstrips - edges) * p.nblocks;
+  [[maybe_unused]] bool redo = false;  // the warp's sums are not finite, and it owns halo cells
   T acc[NL][NP], hi[NL][NP], lo[NL][NP];
 #pragma unroll
   for (int l = 0; l < NL; ++l)
@@ -149,12 +230,9 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
     for (int t = 0; t < NP; ++t) acc[l][t] = hi[l][t] = lo[l][t] = T(0);
 
   if (busy) {
-    const bool first = gw < edge_items;
-    const int strip = first ? (gw % edges ? p.nstrips - 1 : 0) : 1 + (int)((gw - edge_items) % (p.nstrips - edges));
-    const int blk = first ? (int)(gw / edges) : (int)((gw - edge_items) / (p.nstrips - edges));
-    const int sl = first ? p.sl_e : p.sl, nblocks = first ? p.nblocks_e : p.nblocks;
-    const int cs = R + strip * AP::WOUT, ce = min(cs + AP::WOUT, p.d1 - R);
-    const int own_lo = strip == 0 ? 0 : cs, own_hi = strip == p.nstrips - 1 ? p.d1 : ce;
+    const AdjItem it = adj_item<ST, AP>(p, gw);
+    const int cs = it.cs, ce = it.ce, own_lo = it.own_lo, own_hi = it.own_hi;
+    const int i0 = it.i0, i1 = it.i1, o0 = it.o0, o1 = it.o1;
     const int el = cs + p.shift - AP::ML + lane * V;
     const int col0 = el - p.shift;
     const int w0 = cs - AP::ML;                   // column of the window's element 0
@@ -167,8 +245,6 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
       inner[e] = col0 + e >= R && col0 + e < p.d1 - R;
       own[e] = col0 + e >= own_lo && col0 + e < own_hi;
     }
-    const int i0 = R + blk * sl, i1 = min(i0 + sl, p.d0 - R);
-    const int o0 = blk == 0 ? 0 : i0, o1 = blk == nblocks - 1 ? p.d0 : i1;  // rows owned
     const int pstart = AP::FILL ? o0 + R - AP::NFILL * NPH : max(0, o0 - B * R), pend = min(p.d0, o1 + B * R);
     const int ng = (o1 + B * R - pstart + NPH - 1) / NPH;
     // rows [fast_lo, fast_hi): every row that enters or leaves a level is interior
@@ -343,7 +419,9 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
           pair_add(hi[l][t], lo[l][t], acc[l][t]);
           hi[l][t] = mine ? hi[l][t] : T(0);
           lo[l][t] = mine ? lo[l][t] : T(0);
+          redo = redo || !(hi[l][t] - hi[l][t] == T(0));
         }
+      redo = __any_sync(0xffffffffu, redo) && it.rim;
     }
   }
   if constexpr (COEF) {
@@ -358,6 +436,12 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
         part_hi[l * NT + t][threadIdx.x] = hi[l][t];
         part_lo[l * NT + t][threadIdx.x] = lo[l][t];
       }
+    if (redo) {
+      static_assert(NL <= 2, "recount forms lam^0 and lam^1");
+#pragma unroll 1
+      for (int k = 0; k < NL * NT; ++k)
+        recount<ST, AP>(p, gw, k / NT, k % NT, part_hi[k][threadIdx.x], part_lo[k][threadIdx.x]);
+    }
     __syncthreads();
     for (int k = wid; k < NL * NT; k += kWarps) {
       T h = part_hi[k][lane], c = part_lo[k][lane];
@@ -372,7 +456,7 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
         pair_add(h, c, h2);
         c = Arith<T>::add(c, c2);
       }
-      if (lane == 0) sums[k] = (double)h + (double)c;
+      if (lane == 0) sums[k] = (double)h + (h - h == T(0) ? (double)c : 0.0);  // c is NaN beside an infinite h
     }
     __syncthreads();
     static_assert(NT <= kWarps * 32, "a thread per term");
