@@ -361,10 +361,11 @@ __global__ void __launch_bounds__(kGradWarps * 32)
           dn[e] = vedge && inner[e] ? A::sub(x[e], u1[e]) : T(0);
           sn[e] = A::mul(dn[e], dn[e]);
           const T s = A::add(A::add(A::add(A::add(eps, sv[e]), sn[e]), sh[e]), e > 0 ? sh[e > 0 ? e - 1 : 0] : sleft);
-          const T q = rsqrt_near(s);
           const bool in = row_in && inner[e];
           const T lv = in ? l1[e] : T(0);
-          w1[e] = in ? A::mul(A::mul(A::mul(num, lv), q), A::mul(q, q)) : T(0);
+          T q;
+          const T w = rsqrt_cube(A::mul(num, lv), s, q);
+          w1[e] = in ? w : T(0);
           l1[e] = lv;
           if (want_coef && in && sum_col[e] && pp - 1 >= i0 && pp - 1 < i1) pnum += (double)A::mul(lv, q);
         }
