@@ -363,11 +363,13 @@ __global__ void __launch_bounds__(kGradWarps * 32)
           const T s = A::add(A::add(A::add(A::add(eps, sv[e]), sn[e]), sh[e]), e > 0 ? sh[e > 0 ? e - 1 : 0] : sleft);
           const bool in = row_in && inner[e];
           const T lv = in ? l1[e] : T(0);
-          T q;
-          const T w = rsqrt_cube(A::mul(num, lv), s, q);
+          T y, res;
+          rsqrt_split(s, y, res);
+          const T w = rsqrt_cube(A::mul(num, lv), y, res);
           w1[e] = in ? w : T(0);
           l1[e] = lv;
-          if (want_coef && in && sum_col[e] && pp - 1 >= i0 && pp - 1 < i1) pnum += (double)A::mul(lv, q);
+          if (want_coef && in && sum_col[e] && pp - 1 >= i0 && pp - 1 < i1)
+            pnum += (double)A::mul(lv, rsqrt_of(y, res));
         }
         // fluxes: horizontal edges of row p-1, vertical edges between rows p-2 and p-1
         const T wafter = row_elem<V, V>(w1);

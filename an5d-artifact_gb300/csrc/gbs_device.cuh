@@ -290,28 +290,34 @@ __device__ __forceinline__ bool rsqrt_range(double s) {
 __device__ __noinline__ inline double rsqrt_rare(double s) { return 1.0 / sqrt(s); }
 // 1/sqrt(s) to about one rounding
 __device__ __forceinline__ double rsqrt_near(double s) { return rsqrt_range(s) ? rsqrt_core(s) : rsqrt_rare(s); }
-// y ~ 1/sqrt(s) and e = 1 - s y^2, so that 1/sqrt(s) = y (1 + e/2) and its cube
-// y^3 (1 + 3 e/2) to about 2^-44 (e is near 2^-22)
+
+// The same as a root y and its residual e = 1 - s y^2, for results that use it
+// more than once: 1/sqrt(s) = y (1 - e)^(-1/2). In double y is the root above
+// and e is left at 0; in float y is the hardware's estimate and e, about 2^-22,
+// is exact to first order (the product s y is kept whole).
+__device__ __forceinline__ void rsqrt_split(double s, double &y, double &e) {
+  y = rsqrt_near(s);
+  e = 0.0;
+}
 __device__ __forceinline__ void rsqrt_split(float s, float &y, float &e) {
   y = rsqrtf(s);
   const float p = __fmul_rn(s, y);
   e = __fmaf_rn(-p, y, 1.0f);
-  e = __fmaf_rn(-__fmaf_rn(s, y, -p), y, e);  // the product s y exact
+  e = __fmaf_rn(-__fmaf_rn(s, y, -p), y, e);
   if (!(s > 0.0f && s < 3e38f)) e = 0.0f;
 }
-// q = 1/sqrt(s) rounded; returns x q^3
-__device__ __forceinline__ double rsqrt_cube(double x, double s, double &q) {
-  q = rsqrt_near(s);
-  return __dmul_rn(__dmul_rn(x, q), __dmul_rn(q, q));
+// the root itself
+__device__ __forceinline__ double rsqrt_of(double y, double) { return y; }
+__device__ __forceinline__ float rsqrt_of(float y, float e) { return __fmaf_rn(__fmul_rn(0.5f, y), e, y); }
+// x times the root's cube, x y^3 (1 - e)^(-3/2). In float the rounded root's
+// error would enter three times: the gradient of gradient2d, one step, against
+// 64 bits, as a share of the error with the root in double and rounded, 0.80
+// to 0.93 (with the rounded root 1.12 on smooth grids). In double the residual
+// would have to leave the range test's branch as well: 8% of the step.
+__device__ __forceinline__ double rsqrt_cube(double x, double y, double) {
+  return __dmul_rn(__dmul_rn(x, y), __dmul_rn(y, y));
 }
-// In float the cube of the unrounded root: q's rounding error would enter three
-// times. The gradient of gradient2d, one step, against 64 bits, as a share of
-// the error with the root in double and rounded: 0.80 to 0.93 (with q 1.12 on
-// smooth grids).
-__device__ __forceinline__ float rsqrt_cube(float x, float s, float &q) {
-  float y, e;
-  rsqrt_split(s, y, e);
-  q = __fmaf_rn(__fmul_rn(0.5f, y), e, y);
+__device__ __forceinline__ float rsqrt_cube(float x, float y, float e) {
   const float t = __fmul_rn(__fmul_rn(x, y), __fmul_rn(y, y));
   return __fmaf_rn(t, __fmul_rn(1.5f, e), t);
 }
