@@ -291,6 +291,7 @@ __global__ void __launch_bounds__(kGradWarps * 32)
     const int el = cs + g.shift - GP::ML + lane * V;
     const int col0 = el - g.shift;
     const bool in_row = el >= 0 && el + V <= g.pitch;
+    const bool edge = cs - GP::ML < R || cs - GP::ML + GP::COLS > g.d1 - R;
     bool inner[V], hedge[V], sum_col[V];  // hedge: an end of the edge to column e + 1 is an interior column
     bool whole = true;
 #pragma unroll
@@ -345,20 +346,22 @@ __global__ void __launch_bounds__(kGradWarps * 32)
         ld_vec<T, V>(lx, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB + 512));
         const bool row_in = pp - 1 >= R && pp - 1 < g.d0 - R;  // row p-1 is interior
         const bool vedge = pp >= R && pp - 1 < g.d0 - R;       // row p-1 or row p is
+        const bool rim = edge || !row_in || !vedge;
         // horizontal edges of row p-1 (e: between columns e and e+1)
         T dh[V], sh[V];
         const T after = row_elem<V, V>(u1);
 #pragma unroll
         for (int e = 0; e < V; ++e) {
           dh[e] = A::sub(e + 1 < V ? u1[e + 1 < V ? e + 1 : e] : after, u1[e]);
-          dh[e] = row_in && hedge[e] ? dh[e] : T(0);
+          if (rim) dh[e] = row_in && hedge[e] ? dh[e] : T(0);
           sh[e] = A::mul(dh[e], dh[e]);
         }
         const T sleft = shfl_up(sh[V - 1], 1);
         T dn[V], sn[V], w1[V];
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          dn[e] = vedge && inner[e] ? A::sub(x[e], u1[e]) : T(0);
+          dn[e] = A::sub(x[e], u1[e]);
+          if (rim) dn[e] = vedge && inner[e] ? dn[e] : T(0);
           sn[e] = A::mul(dn[e], dn[e]);
           const T s = A::add(A::add(A::add(A::add(eps, sv[e]), sn[e]), sh[e]), e > 0 ? sh[e > 0 ? e - 1 : 0] : sleft);
           const bool in = row_in && inner[e];
