@@ -30,6 +30,7 @@
 #include <mutex>
 #include <vector>
 
+#include "batch_blocks.h"
 #include "engine_internal.h"
 #include "kernel2d.cuh"
 
@@ -228,62 +229,12 @@ int family_degree(int sid) {
   }
 }
 
-// time blocks of T steps: blocks of degree bs plus single steps, with as
-// many blocks as T has parity (launch k reads plane k%2)
-std::vector<int> batch_blocks(int T, int bs) {
-  std::vector<int> out;
-  if (T <= 0) return out;
-  int n = T / bs, r = T - n * bs;
-  if (((n + r) - T) % 2 != 0) {  // only possible for even bs
-    if (n > 0) {
-      --n;
-      r += bs;
-    }
-  }
-  for (int i = 0; i < n; ++i) out.push_back(bs);
-  for (int i = 0; i < r; ++i) out.push_back(1);
-  return out;
-}
-
 // degree of the layered schedule's full blocks
 int layered_degree(int sid) {
   const Picks &p = batch_picks(sid, kFma ? 1 : 0);
   int b = 0;
   while (b < kBatchMaxB && p.lb[b + 1]) ++b;
   return b;
-}
-
-// Time blocks of T steps for the layered schedule: what is left over by full
-// blocks of bs steps first, so that the grids of a stencil soon run at the
-// same degree, then the full blocks; as many blocks as T has parity (launch k
-// reads plane k%2), for which the rest, or a full block, is split in two.
-// For odd T the last block has the steps that batch_blocks gives it: the plane
-// without the result keeps the state before it, from which a run of odd T that
-// is repeated starts, under every schedule.
-std::vector<int> layered_blocks(int T, int bs, int persistent_bs) {
-  std::vector<int> out;
-  if (T <= 0 || bs < 1) return out;
-  const int last = T % 2 ? batch_blocks(T, persistent_bs).back() : 0;
-  T -= last;  // an even rest
-  int full = T / bs;
-  const int rest = T - full * bs;
-  auto halves = [&](int x) {
-    out.push_back((x + 1) / 2);
-    out.push_back(x / 2);
-  };
-  if (T == 0) {
-  } else if ((full + (rest > 0) - T) % 2 == 0) {
-    if (rest > 0) out.push_back(rest);
-  } else if (rest >= 2) {
-    halves(rest);
-  } else {  // a full block goes, and one or three blocks take its steps
-    --full;
-    halves(bs);
-    if (rest > 0) out.push_back(rest);
-  }
-  out.insert(out.end(), full, bs);
-  if (last > 0) out.push_back(last);
-  return out;
 }
 }  // namespace
 }  // namespace gbs
@@ -367,6 +318,11 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
                                           : batch_blocks(bg.timestep, family_degree(bg.stencil));
     if (bg.timestep > 0 && blocks[g].empty())
       return fail(GBS_ERR_UNSUPPORTED, "batch grid %d: no batched kernels built for %s", g, s->name);
+    // the last block of an odd T takes the persistent schedule's degree, which
+    // the layered launchers of the stencil must reach
+    for (int b : blocks[g])
+      if (mode == GBS_BATCH_LAYERED && (b > kBatchMaxB || !batch_picks(bg.stencil, kFma ? 1 : 0).lb[b]))
+        return fail(GBS_ERR_UNSUPPORTED, "batch grid %d: no batched kernel of degree %d built for %s", g, b, s->name);
     cells += (long long)bg.n[0] * bg.n[1] * bg.timestep;
     // validate every strip window of every degree used
     for (size_t k = 0; k < blocks[g].size(); ++k) {
