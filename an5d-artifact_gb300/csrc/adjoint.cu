@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kGradWarps * 32)
         ld_vec<T, V>(lx, reinterpret_cast<const T *>(my + rd + ph * GP::ROWB + 512));
         const bool row_in = pp - 1 >= R && pp - 1 < g.d0 - R;  // row p-1 is interior
         const bool vedge = pp >= R && pp - 1 < g.d0 - R;       // row p-1 or row p is
-        const bool rim = edge || !row_in || !vedge;
+        const bool rim = edge || !row_in;
         // horizontal edges of row p-1 (e: between columns e and e+1)
         T dh[V], sh[V];
         const T after = row_elem<V, V>(u1);

@@ -423,7 +423,7 @@ gbs_status validate3d(const Layout &L, const Geometry3D &g) {
 gbs_status validate2d(const Layout &L, const Geometry2D &g) {
   const int R = L.rad, V = L.V;
   if (g.wout <= 0) return fail(GBS_ERR_UNSUPPORTED, "fused degree %d leaves no output columns", g.b);
-  if (L.shift % 1 != 0 || (L.pitch * (long long)L.esize) % 16 != 0)
+  if ((L.pitch * (long long)L.esize) % 16 != 0)
     return fail(GBS_ERR_INVALID, "internal: row pitch not 16-byte aligned");
   for (int s = 0; s < g.nstrips; ++s) {
     const int cs = R + s * g.wout;
@@ -632,14 +632,9 @@ gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash,
 // writes them, divisor and eps resolved, sl 0 = the planner's choice.
 gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                         int b, const void *src, void *dst, cudaStream_t stream, int *err) {
-  return launch_block_stash(d, L, coef, div, eps, sl, b, src, dst, nullptr, stream, err);
-}
-
-gbs_status launch_block_stash(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
-                              int b, const void *src, void *dst, void *stash, cudaStream_t stream, int *err) {
   BlockPlan plan;
-  gbs_status st = plan_block(d, L, coef, div, eps, sl, b, stash != nullptr, err, &plan);
-  return st == GBS_OK ? launch_plan(plan, src, dst, stash, stream, false) : st;
+  gbs_status st = plan_block(d, L, coef, div, eps, sl, b, false, err, &plan);
+  return st == GBS_OK ? launch_plan(plan, src, dst, nullptr, stream, false) : st;
 }
 }  // namespace gbs
 

@@ -54,10 +54,10 @@ std::vector<int> split_steps(int T, int bt);
 // The launches of d's time loop at degree bt: split_steps, but for odd T the
 // last launch takes the steps that the degree of tuned_last would give it.
 std::vector<int> loop_steps(const gbs_desc *d, int bt);
-// resident_warps: warps the GPU holds at once for this kernel (0 = unknown)
-// rows per stream block of a 2-D launch of nstrips strips over ni rows whose
-// blocks overlap by br rows at each end
 int sm_count();
+// rows per stream block of a 2-D launch of nstrips strips over ni rows whose
+// blocks overlap by br rows at each end; resident_warps: warps the GPU holds at
+// once for this kernel (0 = unknown)
 int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps);
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident_warps);
 long long resident_warps_2d(int sid, int dtype, int fma, int b);
@@ -78,18 +78,15 @@ struct BlockPlan {
   Launch3D a3;
   Launch3DFn f3;
 };
-// `coef` must outlive the plan
+// `coef` must outlive the plan. stash: the launch also stores the states after
+// 1 .. b-1 steps (interior cells) to the planes stash, stash + plane, ... (2-D
+// grids)
 gbs_status plan_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl, int b,
                       bool stash, int *err, BlockPlan *out);
 // pdl: the stream's previous operation is a stencil launch (see Launch2D::pdl)
 gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream, bool pdl);
 gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                         int b, const void *src, void *dst, cudaStream_t stream, int *err);
-// launch_block that also stores the states after 1 .. b-1 steps (interior
-// cells) to the planes stash, stash + plane, ... (2-D grids only; stash may
-// be null)
-gbs_status launch_block_stash(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
-                              int b, const void *src, void *dst, void *stash, cudaStream_t stream, int *err);
 // the layered batched launchers of a stencil (Picks::lb) and their row costs
 const Picks &batch_picks(int sid, int fma);
 int max_bt(int sid, int dtype, int fma);
