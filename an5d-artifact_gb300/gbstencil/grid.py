@@ -22,7 +22,7 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def current_stream(device) -> int:
-    if _raw_stream is None:
+    if _raw_stream is None or device.type != "cuda":  # (a grid on another device is refused there)
         return torch.cuda.current_stream(device).cuda_stream
     index = device.index
     return _raw_stream(torch.cuda.current_device() if index is None else index)
