@@ -152,7 +152,6 @@ template <class ST, typename T>
 __global__ void __launch_bounds__(kAdjThreads) halo_kernel(const __grid_constant__ AdjGeom g, const T *lam, T *hg,
                                                            const __grid_constant__ LinCoef<T, ST::kTerms> cf) {
   constexpr int R = ST::kRad, W = 2 * R + 1;
-  wait_for_previous();
   const HaloPlan hp = halo_plan(g);
   int i, j, c;
   if (!halo_cell(g, hp, (long long)blockIdx.x * kAdjThreads + threadIdx.x, i, j, c)) return;
@@ -187,7 +186,6 @@ __global__ void __launch_bounds__(kAdjThreads) coef_kernel(const __grid_constant
                                                            double *part, T inv_div) {
   constexpr int NT = ST::kTerms;
   constexpr int SEG = 128;
-  wait_for_previous();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int R = g.rad;
   const int width = g.last - 2 * R;
@@ -280,7 +278,6 @@ __global__ void __launch_bounds__(kGradWarps * 32)
   static_assert(ST::kKind != KIND_GRADIENT || ST::kRad == 1, "radius 1");
   __shared__ __align__(128) unsigned char smem[kGradWarps * GP::RING];
   __shared__ double red[kGradWarps];
-  wait_for_previous();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long gw = item0 + (long long)blockIdx.x * kGradWarps + wid;
   double pnum = 0.0;
@@ -579,10 +576,10 @@ bool transposed_coefficients(const gbs_stencil_def_t *s, const std::vector<doubl
 
 // kernels of one stencil and dtype
 struct AdjKernels {
-  cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t, bool);
-  cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t, bool);
+  cudaError_t (*halo)(const AdjGeom &, const void *, void *, const std::vector<double> &, double, cudaStream_t);
+  cudaError_t (*coef)(const AdjGeom &, const void *, const void *, double *, double, cudaStream_t);
   cudaError_t (*grad)(const AdjGeom &, const void *, const void *, void *, void *, double *, double, double, bool,
-                      cudaStream_t, bool);
+                      cudaStream_t);
 };
 
 // one thread per halo cell of the interior rows, one warp per segment of an all-halo row
@@ -608,35 +605,33 @@ cudaError_t copy_halo(int dtype, const AdjGeom &g, const void *src, void *dst, i
 
 template <class ST, typename T>
 cudaError_t run_halo(const AdjGeom &g, const void *lam, void *hg, const std::vector<double> &coef, double div,
-                     cudaStream_t s, bool pdl) {
+                     cudaStream_t s) {
   if constexpr (ST::kKind == KIND_GRADIENT) {
     return cudaErrorInvalidValue;
   } else {
     LinCoef<T, ST::kTerms> cf;
     const double dv = ST::kHasDiv ? div : 1.0;
     for (int t = 0; t < ST::kTerms; ++t) cf.c[t] = (T)(coef[t] / dv);
-    return launch_kernel(halo_kernel<ST, T>, halo_grid(g), kAdjThreads, 0, s, pdl, g, static_cast<const T *>(lam),
+    return launch_kernel(halo_kernel<ST, T>, halo_grid(g), kAdjThreads, 0, s, g, static_cast<const T *>(lam),
                          static_cast<T *>(hg), cf);
   }
 }
 
 template <class ST, typename T>
-cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *part, double div, cudaStream_t s,
-                     bool pdl) {
+cudaError_t run_coef(const AdjGeom &g, const void *lam, const void *u, double *part, double div, cudaStream_t s) {
   if constexpr (ST::kKind == KIND_GRADIENT || ST::kTerms > kMaxCoefGrad) {
     return cudaErrorInvalidValue;
   } else {
     const double dv = ST::kHasDiv ? div : 1.0;
     const int wave = std::min(kAdjPartRows, adj_wave(reinterpret_cast<const void *>(coef_kernel<ST, T>), kAdjThreads, 0));
-    return launch_kernel(coef_kernel<ST, T>, (unsigned)wave, kAdjThreads, 0, s, pdl, g, static_cast<const T *>(lam),
+    return launch_kernel(coef_kernel<ST, T>, (unsigned)wave, kAdjThreads, 0, s, g, static_cast<const T *>(lam),
                          static_cast<const T *>(u), part, (T)(1.0 / dv));
   }
 }
 
-// pdl: the stream's previous operation is another step (see Launch2D::pdl)
 template <class ST, typename T>
 cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam_out, void *hg, double *part,
-                     double num, double eps, bool want_coef, cudaStream_t s, bool pdl) {
+                     double num, double eps, bool want_coef, cudaStream_t s) {
   if constexpr (ST::kKind != KIND_GRADIENT) {
     return cudaErrorInvalidValue;
   } else {
@@ -654,7 +649,7 @@ cudaError_t run_grad(const AdjGeom &g, const void *u, const void *lam, void *lam
     for (long long item0 = 0; item0 < items; item0 += most) {
       const unsigned grid = (unsigned)((std::min(most, items - item0) + kGradWarps - 1) / kGradWarps);
       const cudaError_t e =
-          launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, pdl || item0 > 0, g,
+          launch_kernel(grad2d_kernel<ST, T>, grid, kGradWarps * 32, 0, s, g,
                         static_cast<const T *>(u), static_cast<const T *>(lam), static_cast<T *>(lam_out),
                         static_cast<T *>(hg), part, (T)num, (T)eps, want_coef ? 1 : 0, nstrips, nblocks, sl, item0);
       if (e != cudaSuccess) return e;
@@ -994,8 +989,8 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     return 1;
   };
   // b adjoint steps lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_{t+1-b}), u = the state u_t (u_{t-1} one plane
-  // before it, ...); b > 1 for blocked stencils only. follows: the stream's previous operation is such a step
-  auto steps = [&](const char *u, int b, bool follows) -> gbs_status {
+  // before it, ...); b > 1 for blocked stencils only
+  auto steps = [&](const char *u, int b) -> gbs_status {
     AdjStep2D a{};
     a.g = &g;
     a.lam = lam[cur];
@@ -1005,25 +1000,23 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     a.part = part;
     a.coef = coef.data();
     a.div = sd->divisor ? div : 1.0;
-    a.pdl = follows;
     CK(P2.step[want][b](a, s), "adjoint: 2-D steps");
     cur ^= 1;
     return GBS_OK;
   };
   BlockPlan planT{};  // the transposed step of the stencils that the forward kernels serve
   // one adjoint step lam[cur] (= lam_{t+1}) -> lam[cur ^ 1] (= lam_t) on state u_t
-  auto step = [&](const char *u, bool follows) -> gbs_status {
-    if (blocked) return steps(u, 1, follows);
+  auto step = [&](const char *u) -> gbs_status {
+    if (blocked) return steps(u, 1);
     if (gradient) {
-      CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s, follows),
+      CK(K.grad(g, u, lam[cur], lam[cur ^ 1], hg, part, coef[0], eps, dev_coef_grad != nullptr, s),
          "adjoint: gradient2d step");
     } else {
-      // each of these waits for the one before it and is launched while that ends
-      CK(K.halo(g, lam[cur], hg, coef, div, s, follows), "adjoint: halo");
-      if (dev_coef_grad) CK(K.coef(g, lam[cur], u, part, div, s, true), "adjoint: coefficients");
+      CK(K.halo(g, lam[cur], hg, coef, div, s), "adjoint: halo");
+      if (dev_coef_grad) CK(K.coef(g, lam[cur], u, part, div, s), "adjoint: coefficients");
       gbs_status r = GBS_OK;
       if (planT.dim == 0) r = plan_block(&dT, L, coefT.data(), div, eps, 0, 1, false, err, &planT);
-      if (r == GBS_OK) r = launch_plan(planT, lam[cur], lam[cur ^ 1], nullptr, s, true);
+      if (r == GBS_OK) r = launch_plan(planT, lam[cur], lam[cur ^ 1], nullptr, s);
       if (r != GBS_OK) return r;
     }
     cur ^= 1;
@@ -1034,7 +1027,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
     // no forward state enters: T transposed steps from lam_T
     for (int left = d->timestep; left > 0;) {
       const int b = blocked ? degree(left) : 1;
-      st = blocked ? steps(nullptr, b, left < d->timestep) : step(nullptr, left < d->timestep);
+      st = blocked ? steps(nullptr, b) : step(nullptr);
       if (st != GBS_OK) return st;
       left -= b;
     }
@@ -1071,14 +1064,14 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
                                                                          int top) -> gbs_status {
       const int l = b - a, nfree = w.slots - top;
       if (l <= 0) return GBS_OK;
-      if (l == 1) return step(ua, false);
+      if (l == 1) return step(ua);
       if (nfree == 0) {
         for (int t = b - 1; t > a; --t) {
           gbs_status r = advance(ua, work1, t - a);
-          if (r == GBS_OK) r = step(work1, false);
+          if (r == GBS_OK) r = step(work1);
           if (r != GBS_OK) return r;
         }
-        return step(ua, false);
+        return step(ua);
       }
       const int m = revolve_split(l, nfree);
       char *snap = stash + (size_t)top * w.plane_bytes;
@@ -1160,7 +1153,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
         if (plan.dim == 0) r = plan_block(d, L, coef.data(), div, eps, 0, bb, bb > 1, err, &plan);
         if (r == GBS_OK)
           r = launch_plan(plan, buf + (size_t)(k - 1) * w.plane_bytes, buf + (size_t)(k - 1 + bb) * w.plane_bytes,
-                          bb > 1 ? buf + (size_t)k * w.plane_bytes : nullptr, s2, k > 1);
+                          bb > 1 ? buf + (size_t)k * w.plane_bytes : nullptr, s2);
         if (r != GBS_OK) return r;
         k += bb;
       }
@@ -1178,7 +1171,7 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
       for (int k = c - 1; k >= 0 && st == GBS_OK;) {
         const int bb = blocked ? degree(k + 1) : 1;
         const char *u = buf + (size_t)k * w.plane_bytes;
-        st = blocked ? steps(u, bb, k < c - 1) : step(u, k < c - 1);
+        st = blocked ? steps(u, bb) : step(u);
         k -= bb;
       }
       cudaEventRecord(freed[b], s);

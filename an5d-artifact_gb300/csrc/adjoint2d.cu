@@ -214,7 +214,6 @@ __global__ void __launch_bounds__(kWarps * 32, (AdjPipe2D<ST, B, COEF>::FILL ? 2
   constexpr int NP = COEF ? NT : 1, NL = COEF ? B : 1;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ double sums[NL * NP];
-  wait_for_previous();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const long long gw = p.item0 + (long long)blockIdx.x * kWarps + wid;
   // this CTA's row of the partial sums, read ahead of its update
@@ -557,7 +556,7 @@ template <class ST, int B, bool COEF> cudaError_t launch(const AdjStep2D &a, cud
   const long long most = COEF ? kMost : items;
   for (p.item0 = 0; p.item0 < items; p.item0 += most) {
     const unsigned grid = (unsigned)((std::min(most, items - p.item0) + kWarps - 1) / kWarps);
-    const cudaError_t e = launch_kernel(kern, grid, kWarps * 32, smem, stream, a.pdl || p.item0 > 0, p);
+    const cudaError_t e = launch_kernel(kern, grid, kWarps * 32, smem, stream, p);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;

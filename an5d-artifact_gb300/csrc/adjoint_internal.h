@@ -24,7 +24,6 @@ struct AdjStep2D {
   double *part;          // kAdjPartRows x terms, accumulated (coefficient gradients only)
   const double *coef;    // as the source writes them
   double div;            // the divisor, 1 where there is none
-  bool pdl;              // the stream's previous operation is another step (see Launch2D::pdl)
 };
 using AdjStep2DFn = cudaError_t (*)(const AdjStep2D &, cudaStream_t);
 // launchers of one stencil: [coefficient gradients][degree], null where none is built

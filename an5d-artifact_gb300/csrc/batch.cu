@@ -484,12 +484,10 @@ extern "C++" gbs_status GBS_BATCH_FN(gbs_batch_build)(const gbs_batch_grid *grid
       cudaError_t le = cudaEventRecord(fork, cs);
       for (int k = 0; k < GBS_NUM_STENCILS; ++k)
         if (side[k] && le == cudaSuccess) le = cudaStreamWaitEvent(side[k], fork, 0);
-      int prev = -1;
       for (const Group &q : groups) {
         if (le != cudaSuccess) break;
         le = batch_picks(q.sid, kFma ? 1 : 0)
-                 .lb[q.b](h->d_grids, h->d_items, q.first, q.count, side[q.sid], q.sid == prev);
-        prev = q.sid;
+                 .lb[q.b](h->d_grids, h->d_items, q.first, q.count, side[q.sid]);
         ++h->kernels;
       }
       for (int k = 0; k < GBS_NUM_STENCILS; ++k) {  // join even after a failure, so that the capture can end

@@ -542,9 +542,8 @@ gbs_status run_loop(const gbs_desc *d, const Layout &L, void *dev_A, cudaStream_
     gbs_status st = GBS_OK;
     if (j == 0 || steps[j] != steps[j - 1])
       st = plan_block(d, L, coef.data(), div, eps, sl, steps[j], false, err, &plan);
-    // each launch but the first follows the previous one of this loop on the stream
     if (st == GBS_OK)
-      st = launch_plan(plan, base + (j % 2) * plane_bytes, base + ((j + 1) % 2) * plane_bytes, nullptr, stream, j > 0);
+      st = launch_plan(plan, base + (j % 2) * plane_bytes, base + ((j + 1) % 2) * plane_bytes, nullptr, stream);
     if (st != GBS_OK) return st;
   }
   return GBS_OK;
@@ -610,18 +609,16 @@ gbs_status plan_block(const gbs_desc *d, const Layout &L, const double *coef, do
   return GBS_OK;
 }
 
-gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream, bool pdl) {
+gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream) {
   cudaError_t e;
   if (plan.dim == 2) {
     plan.a2.src = src;
     plan.a2.dst = dst;
     plan.a2.stash = stash;
-    plan.a2.pdl = pdl;
     e = plan.f2(plan.a2, stream);
   } else {
     plan.a3.src = src;
     plan.a3.dst = dst;
-    plan.a3.pdl = pdl;
     e = plan.f3(plan.a3, stream);
   }
   return e == cudaSuccess ? GBS_OK : cuda_fail(e, plan.dim == 2 ? "2-D stencil launch" : "3-D stencil launch");
@@ -634,7 +631,7 @@ gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, 
                         int b, const void *src, void *dst, cudaStream_t stream, int *err) {
   BlockPlan plan;
   gbs_status st = plan_block(d, L, coef, div, eps, sl, b, false, err, &plan);
-  return st == GBS_OK ? launch_plan(plan, src, dst, nullptr, stream, false) : st;
+  return st == GBS_OK ? launch_plan(plan, src, dst, nullptr, stream) : st;
 }
 }  // namespace gbs
 

@@ -83,8 +83,7 @@ struct BlockPlan {
 // grids)
 gbs_status plan_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl, int b,
                       bool stash, int *err, BlockPlan *out);
-// pdl: the stream's previous operation is a stencil launch (see Launch2D::pdl)
-gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream, bool pdl);
+gbs_status launch_plan(BlockPlan &plan, const void *src, void *dst, void *stash, cudaStream_t stream);
 gbs_status launch_block(const gbs_desc *d, const Layout &L, const double *coef, double div, double eps, int sl,
                         int b, const void *src, void *dst, cudaStream_t stream, int *err);
 // the layered batched launchers of a stencil (Picks::lb) and their row costs

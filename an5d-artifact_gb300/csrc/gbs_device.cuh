@@ -56,16 +56,6 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// ---- programmatic dependent launch ---------------------------------------------
-// Waits until the kernel this one was started behind has finished and its
-// writes are visible (returns at once in a plain launch). The kernels never
-// trigger their dependents early: CTAs that start while a grid of fewer than
-// one wave still runs crowd onto its idle SMs and stay there (j2d9pt f64
-// 1777x2500: 101 us a step without an early trigger, 175 with one at the
-// kernel's start, 138 with one at its end); the launch itself still overlaps
-// (star2d1r f32 4096^2, degree 4: 7.8 us a step as plain launches, 7.2).
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)

@@ -472,7 +472,6 @@ __global__ void __launch_bounds__(kWpc2D * 32, gbs_min_ctas(kWpc2D * 32))
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int w = threadIdx.x >> 5;
   const long long gw = (long long)blockIdx.x * kWpc2D + w;
-  wait_for_previous();
   if (gw >= (long long)p.nstrips * p.nblocks) return;
   warp_item2d<ST, T, B, FMA, STASH>(p, (int)(gw % p.nstrips), (int)(gw / p.nstrips),
                                     smem_raw + (size_t)w * Pipe2D<ST, T, B, FMA>::RING);
@@ -525,7 +524,7 @@ cudaError_t launch2d(const Launch2D &a, cudaStream_t stream) {
   p.stash_stride = a.stash_stride;
   const long long warps = (long long)a.nstrips * a.nblocks;
   const long long grid = (warps + kWpc2D - 1) / kWpc2D;
-  return launch_kernel(kern, (unsigned)grid, kWpc2D * 32, smem, stream, a.pdl, p);
+  return launch_kernel(kern, (unsigned)grid, kWpc2D * 32, smem, stream, p);
 }
 
 // Parameters of one item, from its grid's table entry into p (coefficients by
@@ -568,8 +567,8 @@ __global__ void __launch_bounds__(kWpc2D * 32)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int w = threadIdx.x >> 5;
   const long long gw = (long long)blockIdx.x * kWpc2D + w;
-  const bool busy = gw < count;
-  const BatchItem it = busy ? items[gw] : BatchItem{};  // the tables do not change: read ahead of the wait
+  if (gw >= count) return;
+  const BatchItem it = items[gw];
   const BatchGridDev &g = grids[it.grid];
   unsigned char *ring = smem_raw + (size_t)w * Pipe2D<ST, float, B, FMA>::RING;
   if constexpr (SLOT) {
@@ -578,25 +577,22 @@ __global__ void __launch_bounds__(kWpc2D * 32)
     for (int t = threadIdx.x & 31; t < ST::kTerms; t += 32) p.coef[t] = g.coef[t];
     if ((threadIdx.x & 31) == 0) batch_params<ST>(p, g, it.k, it.sl);
     __syncwarp();
-    wait_for_previous();
-    if (busy) warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
+    warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
   } else {
     Params2D<float, ST::kTerms> p;
     batch_params<ST>(p, g, it.k, it.sl);
 #pragma unroll
     for (int t = 0; t < ST::kTerms; ++t) p.coef[t] = g.coef[t];
-    wait_for_previous();
-    if (busy) warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
+    warp_item2d<ST, float, B, FMA>(p, it.strip, it.blk, ring);
   }
 }
 
 template <class ST, int B, bool FMA>
-cudaError_t batch_launch(const BatchGridDev *grids, const BatchItem *items, int first, int count, cudaStream_t stream,
-                         bool pdl) {
+cudaError_t batch_launch(const BatchGridDev *grids, const BatchItem *items, int first, int count, cudaStream_t stream) {
   constexpr size_t smem = smem_bytes2d<ST, float, B, FMA>() + (ST::kTerms > 25 ? kWpc2D * kParamSlot : 0);
   auto kern = batch_family_kernel<ST, B, FMA>;
   if (const cudaError_t e = allow_smem2d(kern, smem); e != cudaSuccess) return e;
-  return launch_kernel(kern, (unsigned)((count + kWpc2D - 1) / kWpc2D), kWpc2D * 32, smem, stream, pdl, grids,
+  return launch_kernel(kern, (unsigned)((count + kWpc2D - 1) / kWpc2D), kWpc2D * 32, smem, stream, grids,
                        items + first, count);
 }
 

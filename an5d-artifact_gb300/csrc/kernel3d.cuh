@@ -206,7 +206,6 @@ __global__ void __launch_bounds__(TJ * 32, gbs_min_ctas(TJ * 32))
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  wait_for_previous();
 
   auto issue = [&](int plane) GBS_INL {  // lane 0 of every warp: this warp's row of `plane`
     const int n = plane - pstart;
@@ -536,7 +535,7 @@ cudaError_t launch3d(const Launch3D &a, cudaStream_t stream) {
     p.nblocks = a.nblocks;
     p.sl = a.sl;
     for (int t = 0; t < ST::kTerms; ++t) p.coef[t] = fold ? (T)(a.coef[t] / a.div) : (T)a.coef[t];
-    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, a.pdl, p);
+    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, p);
   } else {
     Params3D<T, ST::kTerms> p;
     p.src = static_cast<const T *>(a.src);
@@ -557,7 +556,7 @@ cudaError_t launch3d(const Launch3D &a, cudaStream_t stream) {
     p.divmode = !ST::kHasDiv || fold ? 0 : (a.div_proven ? 2 : 1);
     p.div = (T)a.div;
     p.rdiv = div_reciprocal<T>(a.div);
-    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, a.pdl, p);
+    return launch_kernel(kern, (unsigned)grid, NT, smem, stream, p);
   }
 }
 

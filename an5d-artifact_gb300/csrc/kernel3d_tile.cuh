@@ -200,7 +200,6 @@ __global__ void __launch_bounds__(NW * 32, gbs_min_ctas(NW * 32))
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  wait_for_previous();
 
   // thread 0: the whole box of level-0 plane `plane` into its stage
   int issued = pstart;  // thread 0: one past the last plane issued
@@ -450,7 +449,6 @@ __global__ void __launch_bounds__((NW + 1) * 32, gbs_min_ctas((NW + 1) * 32))
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncthreads();
-  wait_for_previous();
 
   if (w == NW) {
     // producer warp: lane 0 issues every plane of the block
