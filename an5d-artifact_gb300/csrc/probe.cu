@@ -85,7 +85,12 @@ __global__ void div_check_f32(float d, float y, int fast, unsigned long long cou
   const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
     const float x = __uint_as_float((unsigned)i);
-    const float a = fast ? gbs::div_by_fast(x, d, y) : gbs::div_by(x, d, y), b = __fdiv_rn(x, d);
+    // the 2-D kernels' form takes a lane's elements at once, the 3-D one's one by one
+    float v[4] = {x, 1.0f, x, 1.0f};
+    if (fast) gbs::div_by_fast(v, d, y);
+    const float b = __fdiv_rn(x, d), c = fast ? v[0] : b;
+    if (__float_as_uint(c) != __float_as_uint(b) && !(isnan(c) && isnan(b))) ++bad;
+    const float a = fast ? gbs::div_by_fast(x, d, y) : gbs::div_by(x, d, y);
     if (__float_as_uint(a) != __float_as_uint(b) && !(isnan(a) && isnan(b))) ++bad;
   }
   if (bad) atomicAdd(mism, bad);
