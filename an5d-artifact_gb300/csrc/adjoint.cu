@@ -830,6 +830,20 @@ int adj_wave(const void *kernel, int threads, size_t smem) {
 
 using namespace gbs;
 
+namespace gbs {
+namespace {
+gbs_status adjoint_forward(const gbs_desc *d, void *dev_A, int checkpoint_every, void *workspace, void *stream,
+                           bool shared);
+// rows per stream block of the forward launches of one of many instances: at
+// least 4 b r (see shared_rows_2d; a whole wave of blocks measured slower here)
+int instance_rows(const gbs_desc *d, const Layout &L, int b) {
+  const int fma = d->fp_mode == GBS_FP_FMA ? 1 : 0;
+  const int own = geometry2d(L, b, 0, resident_warps_2d(d->stencil, d->dtype, fma, b)).sl;
+  return std::min(d->n[0], std::max({own, 8, 4 * b * L.rad}));
+}
+}  // namespace
+}  // namespace gbs
+
 extern "C" {
 
 gbs_status gbs_adjoint_workspace(const gbs_desc *d, int checkpoint_every, size_t *bytes) {
@@ -905,6 +919,15 @@ gbs_status gbs_adjoint_plan_budget(const gbs_desc *d, size_t budget_bytes, int *
 
 gbs_status gbs_adjoint_forward(const gbs_desc *d, void *dev_A, int checkpoint_every, void *workspace,
                                void *stream) {
+  return adjoint_forward(d, dev_A, checkpoint_every, workspace, stream, false);
+}
+}  // extern "C"
+
+namespace gbs {
+namespace {
+// shared: one of many instances side by side
+gbs_status adjoint_forward(const gbs_desc *d, void *dev_A, int checkpoint_every, void *workspace, void *stream,
+                           bool shared) {
   gbs_status st = check_adjoint_args(d, checkpoint_every, workspace);
   if (st != GBS_OK) return st;
   if (!dev_A) return fail(GBS_ERR_INVALID, "dev_A is NULL");
@@ -923,6 +946,11 @@ gbs_status gbs_adjoint_forward(const gbs_desc *d, void *dev_A, int checkpoint_ev
     if (c <= 0) break;
     gbs_desc dc = *d;
     dc.timestep = c;
+    if (shared && L.dim == 2) {
+      gbs_plan_info pi{};
+      if ((st = gbs_plan(&dc, &pi)) != GBS_OK) return st;
+      dc.sl = instance_rows(&dc, L, pi.bt);
+    }
     if ((st = run_loop(&dc, L, dev_A, s, err)) != GBS_OK) return st;
     if (c % 2) CK(cudaMemcpyAsync(A, A + w.plane_bytes, w.plane_bytes, cudaMemcpyDeviceToDevice, s), "adjoint: plane");
   }
@@ -931,15 +959,8 @@ gbs_status gbs_adjoint_forward(const gbs_desc *d, void *dev_A, int checkpoint_ev
   return GBS_OK;
 }
 
-gbs_status gbs_adjoint_backward(const gbs_desc *d, const void *dev_lamT, void *dev_grad_u0, double *dev_coef_grad,
-                                int checkpoint_every, void *workspace, void *stream) {
-  return gbs_adjoint_backward_slots(d, dev_lamT, dev_grad_u0, dev_coef_grad, checkpoint_every,
-                                    2 * std::max(1, checkpoint_every), workspace, stream);
-}
-
-gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, void *dev_grad_u0,
-                                      double *dev_coef_grad, int checkpoint_every, int slots, void *workspace,
-                                      void *stream) {
+gbs_status adjoint_backward(const gbs_desc *d, const void *dev_lamT, void *dev_grad_u0, double *dev_coef_grad,
+                            int checkpoint_every, int slots, void *workspace, void *stream, bool shared) {
   gbs_status st = check_adjoint_args(d, checkpoint_every, workspace);
   if (st != GBS_OK) return st;
   if (slots < 0) return fail(GBS_ERR_INVALID, "slots must be >= 0");
@@ -1150,7 +1171,9 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
         const int bb = std::min(bre, c - k);
         BlockPlan &plan = planR[bb];
         gbs_status r = GBS_OK;
-        if (plan.dim == 0) r = plan_block(d, L, coef.data(), div, eps, 0, bb, bb > 1, err, &plan);
+        if (plan.dim == 0)
+          r = plan_block(d, L, coef.data(), div, eps, shared && L.dim == 2 ? instance_rows(d, L, bb) : 0, bb, bb > 1, err,
+                         &plan);
         if (r == GBS_OK)
           r = launch_plan(plan, buf + (size_t)(k - 1) * w.plane_bytes, buf + (size_t)(k - 1 + bb) * w.plane_bytes,
                           bb > 1 ? buf + (size_t)k * w.plane_bytes : nullptr, s2);
@@ -1193,6 +1216,22 @@ gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, v
   return GBS_OK;
 }
 
+}  // namespace
+}  // namespace gbs
+
+extern "C" {
+gbs_status gbs_adjoint_backward(const gbs_desc *d, const void *dev_lamT, void *dev_grad_u0, double *dev_coef_grad,
+                                int checkpoint_every, void *workspace, void *stream) {
+  return adjoint_backward(d, dev_lamT, dev_grad_u0, dev_coef_grad, checkpoint_every, 2 * std::max(1, checkpoint_every),
+                          workspace, stream, false);
+}
+
+gbs_status gbs_adjoint_backward_slots(const gbs_desc *d, const void *dev_lamT, void *dev_grad_u0,
+                                      double *dev_coef_grad, int checkpoint_every, int slots, void *workspace,
+                                      void *stream) {
+  return adjoint_backward(d, dev_lamT, dev_grad_u0, dev_coef_grad, checkpoint_every, slots, workspace, stream, false);
+}
+
 gbs_status gbs_adjoint_forward_batch(const gbs_desc *descs, int n, void *const *dev_A, int checkpoint_every,
                                      void *const *workspaces, void *stream) {
   if (!descs || n < 1 || !dev_A || !workspaces) return fail(GBS_ERR_INVALID, "adjoint batch: no instances");
@@ -1202,7 +1241,7 @@ gbs_status gbs_adjoint_forward_batch(const gbs_desc *descs, int n, void *const *
     if (!dev_A[i]) return fail(GBS_ERR_INVALID, "adjoint batch: instance %d has no grid", i);
   }
   return on_branches(n, (cudaStream_t)stream, [&](int i, cudaStream_t bs) {
-    return gbs_adjoint_forward(&descs[i], dev_A[i], checkpoint_every, workspaces[i], bs);
+    return adjoint_forward(&descs[i], dev_A[i], checkpoint_every, workspaces[i], bs, n > 1);
   });
 }
 
@@ -1217,8 +1256,8 @@ gbs_status gbs_adjoint_backward_batch(const gbs_desc *descs, int n, const void *
     if (!dev_lamT[i] || !dev_grad_u0[i]) return fail(GBS_ERR_INVALID, "adjoint batch: instance %d lacks a plane", i);
   }
   return on_branches(n, (cudaStream_t)stream, [&](int i, cudaStream_t bs) {
-    return gbs_adjoint_backward(&descs[i], dev_lamT[i], dev_grad_u0[i], dev_coef_grad ? dev_coef_grad[i] : nullptr,
-                                checkpoint_every, workspaces[i], bs);
+    return adjoint_backward(&descs[i], dev_lamT[i], dev_grad_u0[i], dev_coef_grad ? dev_coef_grad[i] : nullptr,
+                            checkpoint_every, 2 * std::max(1, checkpoint_every), workspaces[i], bs, n > 1);
   });
 }
 

@@ -756,25 +756,16 @@ gbs_status build_streams(const gbs_batch_grid *grids, int ngrids, int dtype, int
     if (st != GBS_OK) return st;
     gbs_plan_info pi;
     if ((st = gbs_plan(&d, &pi)) != GBS_OK) return st;
-    // Rows per stream block of a 2-D grid. The planner's choice for a grid that
-    // has the GPU to itself spreads a small one over every SM in blocks of a
-    // few rows; here the branches share the SMs, and short blocks only repeat
-    // more of the overlap. So one wave of blocks, of at least 4 b r rows (40
-    // grids of 180..1000 a side, T <= 100: 1.69 ms; 4.47 with the planner's
-    // blocks, 3.25 with its blocks for 1/16 of a wave, 1.99 and 2.76 with 32
-    // and 64 rows for every grid). GBS_BATCH_SHARE=1: the planner's for this
-    // grid's share of one wave.
+    // the branches share the GPU. GBS_BATCH_SHARE=1: the planner's rows for this
+    // grid's share of one wave
     if (s->dim == 2) {
       const Layout L = make_layout(&d);
-      const int fma = fp_mode == GBS_FP_FMA ? 1 : 0;
-      const long long wave = std::max(1LL, resident_warps_2d(d.stencil, dtype, fma, pi.bt));
       const char *share_env = std::getenv("GBS_BATCH_SHARE");
       if (share_env && share_env[0] == '1') {
+        const long long wave = resident_warps_2d(d.stencil, dtype, fp_mode == GBS_FP_FMA ? 1 : 0, pi.bt);
         d.sl = geometry2d(L, pi.bt, 0, std::max(1LL, wave / nbr)).sl;
       } else {
-        const long long blocks = std::max(1LL, wave / geometry2d(L, pi.bt, 1, wave).nstrips);
-        const int rows = (int)((d.n[0] + blocks - 1) / blocks);
-        d.sl = std::min(d.n[0], std::max({rows, 8, 4 * pi.bt * s->rad}));
+        d.sl = shared_rows_2d(&d, L, pi.bt);
       }
       if ((st = gbs_plan(&d, &pi)) != GBS_OK) return st;
     }

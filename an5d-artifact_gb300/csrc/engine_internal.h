@@ -61,6 +61,9 @@ int sm_count();
 int stream_rows_2d(int nstrips, int ni, int br, bool f64, long long resident_warps);
 Geometry2D geometry2d(const Layout &L, int b, int sl_req, long long resident_warps);
 long long resident_warps_2d(int sid, int dtype, int fma, int b);
+// rows per stream block of a 2-D grid's launches of degree b where many grids'
+// launches share the GPU
+int shared_rows_2d(const gbs_desc *d, const Layout &L, int b);
 // output columns per strip of the 2-D kernels (Pipe2D::WOUT): the window loses
 // b*r columns on the right and b*r rounded up to whole lanes on the left
 inline int wout2d(int rad, int b, int V) {
