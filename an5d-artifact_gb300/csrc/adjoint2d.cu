@@ -30,9 +30,9 @@
 // launches (a chunk reversed by the binomial schedule takes single steps).
 //
 // Bound: memory latency and instruction issue (a step of a 2048^2 grid moves
-// 50 MB, mostly within the L2). Measured (GB300, j2d5pt f32 2048^2): with
-// products 9.7 us a step in launches of two, without 3.7 in launches of four;
-// the kernel of one step this replaced took 10.5 and 8.6.
+// 50 MB, mostly within the L2; issue 52% busy at 0.73 waves). Measured (GB300,
+// j2d5pt f32 2048^2, cold L2): with products 21.3 us a launch of two steps; the
+// kernel of one step this replaced took 13.0.
 //
 // Built per stencil and element type with -DGBS_SID=<table id>
 // -DGBS_T=<float|double> -DGBS_PICK=<exported name>; a divisor is folded into

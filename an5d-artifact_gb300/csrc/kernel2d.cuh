@@ -459,13 +459,14 @@ template <class ST, typename T, int B, bool FMA> constexpr size_t smem_bytes2d()
 }
 
 // Bound: instruction issue at degree 2 and above for float (HBM at degree 1),
-// the FP64 pipe for double. A row of star2d1r at degree 4 takes 122 warp
-// instructions for its 80 multiplies and FMAs; with one bulk copy per row,
-// its mbarrier wait, vote and elected refill it took 191. Measured (GB300,
-// time per step at the tuned degree, before -> after): star2d1r f32 4096^2
-// 13.2 us (degree 4) -> 6.5 (7); j2d5pt f32 16384^2 125 -> 79; box2d2r f32
-// 3001x2217 24.5 -> 13.1; j2d9pt f64 1777x2500 132 (2) -> 85 (1);
-// j2d9pt-gol f32 1500^2, exact mode, 12.8 -> 9.9.
+// the FP64 pipe for double. A row of star2d1r at degree 4 takes 123 warp
+// instructions for its 80 multiplies and FMAs (degree 7: 202 for 140), issued
+// 73% of the time; with one bulk copy per row, its mbarrier wait, vote and
+// elected refill it took 191. Measured (GB300, time per step at the tuned
+// degree, with those copies -> here): star2d1r f32 4096^2 13.2 us (degree 4) ->
+// 6.7 (8); j2d5pt f32 16384^2 125 -> 80; box2d2r f32 3001x2217 24.5 -> 11.7;
+// j2d9pt f64 1777x2500 132 (2) -> 84 (1; its FP64 pipe 92% busy); j2d9pt-gol
+// f32 1500^2, exact mode, 12.8 -> 6.6.
 template <class ST, typename T, int B, bool FMA, bool STASH = false>
 __global__ void __launch_bounds__(kWpc2D * 32, gbs_min_ctas(kWpc2D * 32))
     stencil2d_kernel(const __grid_constant__ Params2D<T, ST::kTerms> p) {
@@ -559,7 +560,7 @@ static_assert(sizeof(Params2D<float, kBatchMaxTerms>) <= kParamSlot, "parameter 
 // stencils need not wait for each other; one kernel that dispatched on the
 // stencil ran every variant at 128 registers and each layer as long as its
 // slowest item: 48 grids of 128..2048 cells a side, up to 128 steps,
-// 9.0 ms -> 4.1 (GB300); the 512-grid mix of the benchmark 370 -> 718 GCells/s.
+// 9.0 ms -> 4.1 (GB300); the 512-grid mix of the benchmark 370 -> 690 GCells/s.
 template <class ST, int B, bool FMA>
 __global__ void __launch_bounds__(kWpc2D * 32)
     batch_family_kernel(const BatchGridDev *__restrict__ grids, const BatchItem *__restrict__ items, int count) {
