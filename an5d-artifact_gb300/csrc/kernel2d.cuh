@@ -466,7 +466,7 @@ template <class ST, typename T, int B, bool FMA> constexpr size_t smem_bytes2d()
 // degree, with those copies -> here): star2d1r f32 4096^2 13.2 us (degree 4) ->
 // 6.7 (8); j2d5pt f32 16384^2 125 -> 80; box2d2r f32 3001x2217 24.5 -> 11.7;
 // j2d9pt f64 1777x2500 132 (2) -> 84 (1; its FP64 pipe 92% busy); j2d9pt-gol
-// f32 1500^2, exact mode, 12.8 -> 6.6.
+// f32 2048^2, exact mode, 22.4 (1) -> 8.8 (4).
 template <class ST, typename T, int B, bool FMA, bool STASH = false>
 __global__ void __launch_bounds__(kWpc2D * 32, gbs_min_ctas(kWpc2D * 32))
     stencil2d_kernel(const __grid_constant__ Params2D<T, ST::kTerms> p) {

@@ -151,7 +151,7 @@ gbs_status gbs_plan(const gbs_desc *d, gbs_plan_info *out);
  * loop plane 0 holds the state before that launch, and a program that runs it
  * again from there sees the same states whatever degree the table chooses. */
 typedef struct gbs_tune_candidate {
-  int bt, sl;               /* sl 0: the engine's one-wave stream length */
+  int bt, sl;               /* sl 0: the planner's stream length */
   double redundancy;        /* computed / useful cells per launch */
   double model_ms_per_step; /* the model's time for one timestep */
   double ms_per_step;       /* measured; < 0 if the model pruned it */
